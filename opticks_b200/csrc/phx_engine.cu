@@ -68,13 +68,16 @@ struct DevBuf {
 // scratch of the hit merge (grow-only, per engine)
 struct PhxMergeWs {
     DevBuf<uint32_t> sel, tcount, val0, val1, head, tsum, hist, pmin, gor, gsum, hin, hout;
-    DevBuf<unsigned long long> key0, key1, amin, key_or;
+    DevBuf<uint32_t> cell, cell_off, cell_blk;     // table form: cell bits, their popcount prefix
+    DevBuf<unsigned long long> key0, key1, amin;
+    DevBuf<PhxMergeRange> range;
     DevBuf<long long> total;
     void release()
     {
         sel.release(); tcount.release(); val0.release(); val1.release(); head.release(); tsum.release(); hist.release();
         pmin.release(); gor.release(); gsum.release(); hin.release(); hout.release();
-        key0.release(); key1.release(); amin.release(); key_or.release(); total.release();
+        cell.release(); cell_off.release(); cell_blk.release(); range.release();
+        key0.release(); key1.release(); amin.release(); total.release();
     }
 };
 
@@ -2157,47 +2160,41 @@ static int merge_read(phx_engine* e, const void* d, size_t bytes, void* h, cudaS
     return 0;
 }
 
+// ordered positions of the records `mask` selects, in w.sel (null with every record selected)
 template <int LITE>
-static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t mask, float tw, uint32_t* out, long long cap,
-                      long long* num_out, cudaStream_t st)
+static int merge_select(PhxMergeWs& w, const uint32_t* in, long long n, uint32_t mask, const uint32_t** sel, cudaStream_t st)
+{
+    *sel = nullptr;
+    if (mask == 0xffffffffu) return 0;
+    const long long nt = (n + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE;
+    PHX_CU(w.total.ensure(2));
+    PHX_CU(w.tcount.ensure((size_t)nt));
+    PHX_CU(w.sel.ensure((size_t)n));
+    k_merge_sel_count<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p);
+    k_block_scan<<<1, 1024, 0, st>>>(w.tcount.p, (int)nt, w.total.p);
+    k_merge_sel_write<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p, w.sel.p);
+    PHX_CU(cudaGetLastError());
+    *sel = w.sel.p;
+    return 0;
+}
+
+// the sort form of merge_impl (phx_merge.cuh) for keys whose range no table holds
+template <int LITE>
+static int merge_sorted(phx_engine* e, const uint32_t* in, long long n, uint32_t mask, float tw, const PhxMergeRange& range, uint32_t* out,
+                        long long cap, long long* num_out, cudaStream_t st)
 {
     PhxMergeWs& w = e->merge;
-    *num_out = 0;
-    if (n == 0) return 0;
-    long long m = n;
     const uint32_t* sel = nullptr;
-    int rc;
-    PHX_CU(w.total.ensure(2));
-    if (mask != 0xffffffffu) {
-        const long long nt = (n + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE;
-        PHX_CU(w.tcount.ensure((size_t)nt));
-        PHX_CU(w.sel.ensure((size_t)n));
-        k_merge_sel_count<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p);
-        k_block_scan<<<1, 1024, 0, st>>>(w.tcount.p, (int)nt, w.total.p);
-        k_merge_sel_write<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p, w.sel.p);
-        PHX_CU(cudaGetLastError());
-        if ((rc = merge_read(e, w.total.p, sizeof(long long), &m, st))) return rc;
-        sel = w.sel.p;
-    }
-    if (m == 0) return 0;
-    const int W = PhxRec<LITE>::W;
+    int rc = merge_select<LITE>(w, in, n, mask, &sel, st);
+    if (rc) return rc;
+    const long long m = (long long)range.count;
     const unsigned grid = (unsigned)std::min<long long>((m + 255) / 256, 148LL * 16);
-    if (tw == 0.f) {                 // selection only, input order
-        *num_out = m;
-        if (m > cap) return phx_fail(-3, "phx_merge_hits: %lld records selected, out_capacity %lld", m, cap);
-        k_merge_gather<LITE><<<(unsigned)std::min<long long>((m * W + 255) / 256, 148LL * 32), 256, 0, st>>>(in, sel, m, out);
-        PHX_CU(cudaGetLastError());
-        return 0;
-    }
+    PHX_CU(w.total.ensure(2));
     PHX_CU(w.key0.ensure((size_t)m)); PHX_CU(w.key1.ensure((size_t)m));
     PHX_CU(w.val0.ensure((size_t)m)); PHX_CU(w.val1.ensure((size_t)m));
-    PHX_CU(w.key_or.ensure(1));
-    PHX_CU(cudaMemsetAsync(w.key_or.p, 0, sizeof(unsigned long long), st));
-    k_merge_keys<LITE><<<grid, 256, 0, st>>>(in, sel, m, tw, w.key0.p, w.val0.p, w.key_or.p);
+    k_merge_keys<LITE><<<grid, 256, 0, st>>>(in, sel, m, tw, w.key0.p, w.val0.p);
     PHX_CU(cudaGetLastError());
-    unsigned long long kor = 0;
-    if ((rc = merge_read(e, w.key_or.p, sizeof(kor), &kor, st))) return rc;
-    // stable LSD radix passes over the key bytes that are non-zero somewhere
+    // stable LSD radix passes over the key bytes up to the largest bucket and identity
     const long long nt = (m + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE;
     PHX_CU(w.hist.ensure((size_t)(256 * nt)));
     unsigned long long* kin = w.key0.p;
@@ -2205,7 +2202,7 @@ static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t m
     uint32_t* vin = w.val0.p;
     uint32_t* vout = w.val1.p;
     for (int b = 0; b < 8; b++) {
-        if (((kor >> (8 * b)) & 0xffull) == 0ull) continue;
+        if (((b < 4 ? range.bk_max : b < 6 ? 0u : range.id_max) >> (8 * (b < 4 ? b : b - 6))) == 0u) continue;
         k_radix_hist<<<(unsigned)nt, 256, 0, st>>>(kin, m, 8 * b, w.hist.p, (int)nt);
         if ((rc = merge_scan(w, w.hist.p, 256 * nt, nullptr, st))) return rc;
         k_radix_scatter<<<(unsigned)nt, 256, 0, st>>>(kin, vin, kout, vout, m, 8 * b, w.hist.p, (int)nt);
@@ -2230,6 +2227,55 @@ static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t m
     k_merge_reduce<LITE><<<grid, 256, 0, st>>>(in, sel, kin, vin, w.head.p, m, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
     k_merge_write<LITE><<<(unsigned)((ng + 255) / 256), 256, 0, st>>>(in, sel, ng, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p, out);
     PHX_CU(cudaGetLastError());
+    return 0;
+}
+
+template <int LITE>
+static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t mask, float tw, uint32_t* out, long long cap,
+                      long long* num_out, cudaStream_t st)
+{
+    PhxMergeWs& w = e->merge;
+    *num_out = 0;
+    if (n == 0) return 0;
+    int rc;
+    if (tw == 0.f) {                 // selection only, input order
+        const int W = PhxRec<LITE>::W;
+        const uint32_t* sel = nullptr;
+        if ((rc = merge_select<LITE>(w, in, n, mask, &sel, st))) return rc;
+        long long m = n;
+        if (sel && (rc = merge_read(e, w.total.p, sizeof(long long), &m, st))) return rc;
+        if (m == 0) return 0;
+        *num_out = m;
+        if (m > cap) return phx_fail(-3, "phx_merge_hits: %lld records selected, out_capacity %lld", m, cap);
+        k_merge_gather<LITE><<<(unsigned)std::min<long long>((m * W + 255) / 256, 148LL * 32), 256, 0, st>>>(in, sel, m, out);
+        PHX_CU(cudaGetLastError());
+        return 0;
+    }
+    // table form, decided on the device: every kernel leaves at once when the range has more cells
+    // than the table, and the sort form takes over after the one host read
+    const unsigned long long most = phx_merge_cells(n);
+    const long long ncw = (long long)(most / 32ull), nblk = ncw / 1024;
+    PHX_CU(w.range.ensure(1));
+    PHX_CU(w.cell.ensure((size_t)ncw)); PHX_CU(w.cell_off.ensure((size_t)ncw)); PHX_CU(w.cell_blk.ensure((size_t)nblk));
+    PHX_CU(w.key0.ensure((size_t)n)); PHX_CU(w.amin.ensure((size_t)n));
+    PHX_CU(w.gor.ensure((size_t)n)); PHX_CU(w.gsum.ensure((size_t)n));
+    if (LITE) PHX_CU(w.pmin.ensure((size_t)n));
+    PHX_CU(cudaMemsetAsync(w.range.p, 0, sizeof(PhxMergeRange), st));
+    const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 8);
+    k_merge_range<LITE><<<std::max(grid, 148u), 256, 0, st>>>(in, n, mask, tw, w.key0.p, w.range.p, w.cell.p, ncw, w.amin.p, w.pmin.p, w.gor.p,
+                                                              w.gsum.p);
+    k_merge_present<<<grid, 256, 0, st>>>(w.key0.p, n, w.range.p, most, w.cell.p);
+    k_merge_rank<<<(unsigned)nblk, 256, 0, st>>>(w.cell.p, w.range.p, most, w.cell_off.p, w.cell_blk.p);
+    k_block_scan<<<1, 1024, 0, st>>>(w.cell_blk.p, (int)nblk, &w.range.p->groups);
+    k_merge_fold<LITE><<<grid, 256, 0, st>>>(in, w.key0.p, n, w.range.p, most, w.cell.p, w.cell_off.p, w.cell_blk.p, w.amin.p, w.pmin.p,
+                                             w.gor.p, w.gsum.p);
+    k_merge_groups<LITE><<<grid, 256, 0, st>>>(in, w.range.p, most, cap, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p, out);
+    PHX_CU(cudaGetLastError());
+    PhxMergeRange range;
+    if ((rc = merge_read(e, w.range.p, sizeof(range), &range, st))) return rc;
+    if (phx_merge_map(range).cells > most) return merge_sorted<LITE>(e, in, n, mask, tw, range, out, cap, num_out, st);
+    *num_out = range.groups;
+    if (range.groups > cap) return phx_fail(-3, "phx_merge_hits: %lld merged records, out_capacity %lld", range.groups, cap);
     return 0;
 }
 

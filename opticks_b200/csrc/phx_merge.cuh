@@ -12,17 +12,29 @@
 //                          hitcount = sum (16 bits)
 //   window 0 : selection only, records in input order
 //
-// The reference sorts with thrust::sort_by_key and folds with thrust::reduce_by_key.  Here:
+// The reference sorts with thrust::sort_by_key and folds with thrust::reduce_by_key.  Every reduction
+// above is associative and commutative over (time, position), so no order is needed to compute it,
+// only the rank of a key among the keys that occur:
+//   1. k_merge_range   keys of the selected records, their count and the ranges of identity and bucket
+//   2. k_merge_present one bit per (identity, bucket) cell of that range, set where a key occurs
+//   3. k_merge_rank    popcount prefix of the bit table: a cell's rank is its group index, and groups
+//                      come out in ascending key order
+//   4. k_merge_fold    atomics of each record into its group: min (time, position), OR, sum
+//   5. k_merge_groups  the representative record of each group with the reduced fields
+// in one go without a host read (the table's size comes from n, the range stays on the device).  1M
+// sphoton records with a fifth selected, 1 ns windows: 79 us a call, against 247 us through the sort
+// (35 launches and three host reads); what is left is six launches and one read at 4-20 us apiece.
+// Ranges whose cells outnumber the table (phx_merge_cells) are left to a stable sort of the keys:
 //   1. ordered selection (ballot + tile offsets)           -> sel[m] input positions
-//   2. keys (u64) and their bitwise OR                     -> passes only over non-zero key bytes
+//   2. keys (u64); passes only over the key bytes in use
 //   3. stable LSD radix sort, 8-bit digits: per-tile digit histograms (digit-major), one scan,
 //      a scatter ranking equal digits by __match_any_sync so every pass is stable
 //   4. group heads + scan -> group index; warp-segmented reductions (__reduce_*_sync over the
 //      lanes of one group) with one atomic per (warp, group): min (time, position), min position,
 //      OR flagmask, sum hitcount
 //   5. one thread per group writes the representative record with the reduced fields
-// Each reduction is associative and picks the record the left fold of reduce_op picks.  Included by
-// phx_engine.cu after DevBuf and PHX_CU.
+// Each form picks the record the left fold of reduce_op picks.  Included by phx_engine.cu after
+// DevBuf and PHX_CU.
 #pragma once
 #include <stdint.h>
 
@@ -53,6 +65,209 @@ __device__ __forceinline__ uint32_t phx_time_unorder(uint32_t o)
     return (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
 }
 
+// ---------------------------------------------------------------- table form
+// Bits of the cell table for n records: 32 per record, and never fewer than 2^24 (2 MB).  The table
+// is cleared and scanned on each call at 4 B per record, an eighth of the least the records cost.
+__host__ __device__ inline unsigned long long phx_merge_cells(long long n)
+{
+    const unsigned long long c = 32ull * (unsigned long long)n;
+    return c < (1ull << 24) ? (1ull << 24) : c < (1ull << 31) ? ((c + 32767ull) & ~32767ull) : (1ull << 31);
+}
+
+// what k_merge_range finds out (zeroed before it); minima are kept as maxima of the complement
+struct PhxMergeRange {
+    uint32_t id_max, id_cmin, bk_max, bk_cmin;
+    unsigned long long count;
+    long long groups;
+};
+
+// the cells of a range: identities x buckets, 0 when nothing was selected
+struct PhxMergeMap {
+    uint32_t id0, bk0, nbk;
+    unsigned long long cells;
+};
+__host__ __device__ inline PhxMergeMap phx_merge_map(const PhxMergeRange& r)
+{
+    PhxMergeMap m;
+    m.id0 = ~r.id_cmin;
+    m.bk0 = ~r.bk_cmin;
+    m.nbk = r.bk_max - m.bk0 + 1u;                   // 0: 2^32 buckets
+    const unsigned long long nb = m.nbk ? (unsigned long long)m.nbk : (1ull << 32);
+    m.cells = r.count ? (unsigned long long)(r.id_max - m.id0 + 1u) * nb : 0ull;
+    return m;
+}
+
+#define PHX_MERGE_NONE 0xffffffffffffffffull         // key of a record that is not selected (identities are 16 bits)
+
+template <int LITE>
+__device__ __forceinline__ unsigned long long phx_merge_key(const uint32_t* r, float tw)
+{
+    const uint32_t id = r[PhxRec<LITE>::ID] & PhxRec<LITE>::IDMASK;
+    const unsigned bucket = static_cast<unsigned>(__uint_as_float(r[PhxRec<LITE>::TIME]) / tw);
+    return ((unsigned long long)id << 48) | (unsigned long long)bucket;
+}
+
+// 1. keys and their ranges; also clears the cell table and the n group slots
+template <int LITE>
+__global__ void __launch_bounds__(256) k_merge_range(const uint32_t* in, long long n, uint32_t mask, float tw, unsigned long long* key,
+                                                     PhxMergeRange* range, uint32_t* cell, long long ncellw, unsigned long long* amin,
+                                                     uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
+{
+    __shared__ uint32_t s_id, s_idc, s_bk, s_bkc, s_cnt;
+    if (threadIdx.x == 0) s_id = s_idc = s_bk = s_bkc = s_cnt = 0u;
+    __syncthreads();
+    const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    for (long long j = at; j < ncellw / 4; j += stride) reinterpret_cast<uint4*>(cell)[j] = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t id = 0u, idc = 0u, bk = 0u, bkc = 0u, cnt = 0u;
+    for (long long j = at; j < n; j += stride) {
+        const uint32_t* r = in + j * PhxRec<LITE>::W;
+        unsigned long long k = PHX_MERGE_NONE;
+        if (mask == 0xffffffffu || (r[PhxRec<LITE>::FLAG] & mask) != 0u) {
+            k = phx_merge_key<LITE>(r, tw);
+            const uint32_t i = (uint32_t)(k >> 48), b = (uint32_t)k;
+            id = max(id, i); idc = max(idc, ~i); bk = max(bk, b); bkc = max(bkc, ~b);
+            cnt++;
+        }
+        key[j] = k;
+        amin[j] = 0xffffffffffffffffull;
+        if (LITE) pmin[j] = 0xffffffffu;
+        gor[j] = 0u;
+        gsum[j] = 0u;
+    }
+    const unsigned FULL = 0xffffffffu;
+    id = __reduce_max_sync(FULL, id); idc = __reduce_max_sync(FULL, idc);
+    bk = __reduce_max_sync(FULL, bk); bkc = __reduce_max_sync(FULL, bkc);
+    cnt = __reduce_add_sync(FULL, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) {
+        atomicMax(&s_id, id); atomicMax(&s_idc, idc); atomicMax(&s_bk, bk); atomicMax(&s_bkc, bkc);
+        atomicAdd(&s_cnt, cnt);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_cnt) {
+        atomicMax(&range->id_max, s_id); atomicMax(&range->id_cmin, s_idc);
+        atomicMax(&range->bk_max, s_bk); atomicMax(&range->bk_cmin, s_bkc);
+        atomicAdd(&range->count, (unsigned long long)s_cnt);
+    }
+}
+
+__device__ __forceinline__ uint32_t phx_merge_cell(const PhxMergeMap& m, unsigned long long k)
+{
+    return ((uint32_t)(k >> 48) - m.id0) * m.nbk + ((uint32_t)k - m.bk0);
+}
+
+// 2. the cells that occur
+__global__ void __launch_bounds__(256) k_merge_present(const unsigned long long* key, long long n, const PhxMergeRange* range,
+                                                       unsigned long long most, uint32_t* cell)
+{
+    const PhxMergeMap m = phx_merge_map(*range);
+    if (m.cells == 0ull || m.cells > most) return;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
+        const unsigned long long k = key[j];
+        if (k == PHX_MERGE_NONE) continue;
+        const uint32_t c = phx_merge_cell(m, k);
+        const uint32_t bit = 1u << (c & 31u);
+        if (!(cell[c >> 5] & bit)) atomicOr(cell + (c >> 5), bit);   // a stale read only costs the atomic
+    }
+}
+
+// 3. popcount prefix of the table, 1024 words a block (offsets within the block, block totals)
+__global__ void __launch_bounds__(256) k_merge_rank(const uint32_t* cell, const PhxMergeRange* range, unsigned long long most,
+                                                    uint32_t* off, uint32_t* blocksum)
+{
+    const PhxMergeMap m = phx_merge_map(*range);
+    const unsigned long long w0 = (unsigned long long)blockIdx.x * 1024ull;
+    if (m.cells > most || w0 * 32ull >= m.cells) {
+        if (threadIdx.x == 0) blocksum[blockIdx.x] = 0u;
+        return;
+    }
+    __shared__ uint32_t wt[8];
+    const uint4 v = reinterpret_cast<const uint4*>(cell)[w0 / 4 + threadIdx.x];
+    const uint32_t c0 = __popc(v.x), c1 = __popc(v.y), c2 = __popc(v.z), s = c0 + c1 + c2 + __popc(v.w);
+    uint32_t inc = s;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += y; }
+    if (lane == 31) wt[wid] = inc;
+    __syncthreads();
+    uint32_t run = inc - s;
+    for (int k = 0; k < wid; k++) run += wt[k];
+    reinterpret_cast<uint4*>(off)[w0 / 4 + threadIdx.x] = make_uint4(run, run + c0, run + c0 + c1, run + c0 + c1 + c2);
+    if (threadIdx.x == 255) blocksum[blockIdx.x] = run + s;
+}
+
+// 4. each record into its group.  Lanes of a warp that share a group are reduced first, so that many
+// records of one group do not queue on its atomics one by one.
+template <int LITE>
+__global__ void __launch_bounds__(256) k_merge_fold(const uint32_t* in, const unsigned long long* key, long long n,
+                                                    const PhxMergeRange* range, unsigned long long most, const uint32_t* cell,
+                                                    const uint32_t* off, const uint32_t* blocksum, unsigned long long* amin,
+                                                    uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
+{
+    const PhxMergeMap m = phx_merge_map(*range);
+    if (m.cells == 0ull || m.cells > most) return;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
+        const long long j = base + lane;
+        const unsigned long long k = j < n ? key[j] : PHX_MERGE_NONE;
+        const bool ok = k != PHX_MERGE_NONE;
+        uint32_t g = 0xffffffffu, tb = 0xffffffffu, fl = 0u, hc = 0u, pos = (uint32_t)j;
+        if (ok) {
+            const uint32_t c = phx_merge_cell(m, k), w = c >> 5;
+            g = blocksum[w >> 10] + off[w] + __popc(cell[w] & ((1u << (c & 31u)) - 1u));
+            const uint32_t* r = in + j * PhxRec<LITE>::W;
+            tb = phx_time_order(r[PhxRec<LITE>::TIME]);
+            fl = r[PhxRec<LITE>::FLAG];
+            hc = r[PhxRec<LITE>::HC] >> 16;
+        }
+        if (!__any_sync(FULL, ok)) continue;
+        const uint32_t peers = __match_any_sync(FULL, g);
+        bool lead = ok;
+        uint32_t pfirst = pos, pm = pos;
+        if (__any_sync(FULL, ok && (peers & (peers - 1u)) != 0u)) {
+            const uint32_t tmin = __reduce_min_sync(peers, tb);
+            pfirst = __reduce_min_sync(peers, tb == tmin ? pos : 0xffffffffu);
+            pm = __reduce_min_sync(peers, pos);
+            fl = __reduce_or_sync(peers, fl);
+            hc = __reduce_add_sync(peers, hc);
+            tb = tmin;
+            lead = ok && __ffs(peers) - 1 == lane;
+        }
+        if (lead) {
+            atomicMin(amin + g, ((unsigned long long)tb << 32) | (unsigned long long)pfirst);
+            if (LITE) atomicMin(pmin + g, pm);
+            atomicOr(gor + g, fl);
+            atomicAdd(gsum + g, hc);
+        }
+    }
+}
+
+// 5. representative record per group with the reduced fields, a 16 B row a thread
+template <int LITE>
+__global__ void __launch_bounds__(256) k_merge_groups(const uint32_t* in, const PhxMergeRange* range, unsigned long long most,
+                                                      long long cap, const unsigned long long* amin, const uint32_t* pmin,
+                                                      const uint32_t* gor, const uint32_t* gsum, uint32_t* out)
+{
+    constexpr int Q = PhxRec<LITE>::W / 4;
+    const long long ng = range->groups;
+    if (phx_merge_map(*range).cells > most || ng > cap) return;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < ng * Q; x += stride) {
+        const long long g = x / Q;
+        const int q = (int)(x - g * Q);
+        const unsigned long long a = amin[g];
+        const long long i = LITE ? (long long)pmin[g] : (long long)(a & 0xffffffffull);
+        uint32_t r[4];
+        for (int w = 0; w < 4; w++) r[w] = in[i * PhxRec<LITE>::W + 4 * q + w];
+        if (LITE) r[PhxRec<LITE>::TIME & 3] = phx_time_unorder((uint32_t)(a >> 32));
+        if (q == PhxRec<LITE>::FLAG / 4) r[PhxRec<LITE>::FLAG & 3] = gor[g];
+        if (q == PhxRec<LITE>::HC / 4) r[PhxRec<LITE>::HC & 3] = (r[PhxRec<LITE>::HC & 3] & 0xffffu) | ((gsum[g] & 0xffffu) << 16);
+        for (int w = 0; w < 4; w++) out[x * 4 + w] = r[w];
+    }
+}
+
+// ---------------------------------------------------------------- sort form
 // 1a. per-tile selected counts
 template <int LITE>
 __global__ void __launch_bounds__(256) k_merge_sel_count(const uint32_t* in, long long n, uint32_t mask, uint32_t* tcount)
@@ -114,24 +329,15 @@ __global__ void k_merge_gather(const uint32_t* in, const uint32_t* sel, long lon
     }
 }
 
-// 2. keys of the selected records; OR of all keys
+// 2. keys of the selected records
 template <int LITE>
-__global__ void k_merge_keys(const uint32_t* in, const uint32_t* sel, long long m, float tw, unsigned long long* key,
-                             uint32_t* val, unsigned long long* key_or)
+__global__ void k_merge_keys(const uint32_t* in, const uint32_t* sel, long long m, float tw, unsigned long long* key, uint32_t* val)
 {
-    unsigned long long acc = 0ull;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (long long)gridDim.x * blockDim.x) {
         const long long i = sel ? (long long)sel[j] : j;
-        const uint32_t* r = in + i * PhxRec<LITE>::W;
-        const uint32_t id = r[PhxRec<LITE>::ID] & PhxRec<LITE>::IDMASK;
-        const unsigned bucket = static_cast<unsigned>(__uint_as_float(r[PhxRec<LITE>::TIME]) / tw);
-        const unsigned long long k = ((unsigned long long)id << 48) | (unsigned long long)bucket;
-        key[j] = k;
+        key[j] = phx_merge_key<LITE>(in + i * PhxRec<LITE>::W, tw);
         val[j] = (uint32_t)j;
-        acc |= k;
     }
-    for (int o = 16; o > 0; o >>= 1) acc |= __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc) atomicOr(key_or, acc);
 }
 
 // 3a. digit histogram per tile, digit-major: hist[d * ntile + tile]
