@@ -104,11 +104,51 @@ __host__ __device__ inline bool phx_csg_base_typecode(unsigned tc)
 
 PHX_D unsigned nd_u(const float4& q, int k) { return __float_as_uint(k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w); }
 
+// ---------------------------------------------------------------- fixed rounding
+// The sphere, zsphere and cylinder leaves and the ray transforms are inlined in several kernels.  Left
+// to the compiler, which sums become fused multiply-adds depends on the code around them, and a
+// last-bit change of one hit ends in another photon history.  So their roundings are written out:
+// products summed left to right, each product after the first fused into the sum.
+PHX_D float fx_dot(const float3& a, const float3& b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x))); }
+PHX_D float fx_dot2(float ax, float ay, float bx, float by) { return __fmaf_rn(ay, by, __fmul_rn(ax, bx)); }
+PHX_D float3 fx_at(const float3& o, float t, const float3& d)
+{
+    return make_float3(__fmaf_rn(t, d.x, o.x), __fmaf_rn(t, d.y, o.y), __fmaf_rn(t, d.z, o.z));
+}
+// A point or a direction through a 4x4 of row-vector convention (v' = v M), and a normal back through
+// the inverse (v' = M v): the middle product first, then the first, the last and the translation.
+PHX_D float fx_mix(float a, float x, float b, float y, float c, float z) { return __fmaf_rn(c, z, __fmaf_rn(a, x, __fmul_rn(b, y))); }
+PHX_D float3 fx_point(const float4* q, const float3& v)
+{
+    return make_float3(__fadd_rn(fx_mix(q[0].x, v.x, q[1].x, v.y, q[2].x, v.z), q[3].x),
+                       __fadd_rn(fx_mix(q[0].y, v.x, q[1].y, v.y, q[2].y, v.z), q[3].y),
+                       __fadd_rn(fx_mix(q[0].z, v.x, q[1].z, v.y, q[2].z, v.z), q[3].z));
+}
+// (the translation times zero is summed too: it decides the sign of a zero component)
+PHX_D float3 fx_dir(const float4* q, const float3& v)
+{
+    return make_float3(__fmaf_rn(q[3].x, 0.f, fx_mix(q[0].x, v.x, q[1].x, v.y, q[2].x, v.z)),
+                       __fmaf_rn(q[3].y, 0.f, fx_mix(q[0].y, v.x, q[1].y, v.y, q[2].y, v.z)),
+                       __fmaf_rn(q[3].z, 0.f, fx_mix(q[0].z, v.x, q[1].z, v.y, q[2].z, v.z)));
+}
+PHX_D float3 fx_normal(const float4* q, const float3& v)
+{
+    return make_float3(__fmaf_rn(q[0].w, 0.f, fx_mix(q[0].x, v.x, q[0].y, v.y, q[0].z, v.z)),
+                       __fmaf_rn(q[1].w, 0.f, fx_mix(q[1].x, v.x, q[1].y, v.y, q[1].z, v.z)),
+                       __fmaf_rn(q[2].w, 0.f, fx_mix(q[2].x, v.x, q[2].y, v.y, q[2].z, v.z)));
+}
+// unit vectors, by the length of fx_dot or of fx_mix
+PHX_D float3 fx_scale(const float3& v, float f) { return make_float3(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f)); }
+PHX_D float3 fx_unit(const float3& v) { return fx_scale(v, 1.0f / sqrtf(fx_dot(v, v))); }
+PHX_D float3 fx_unit_mix(const float3& v) { return fx_scale(v, 1.0f / sqrtf(fx_mix(v.x, v.x, v.y, v.y, v.z, v.z))); }
+// discriminant b b - d c
+PHX_D float fx_disc(float d, float b, float c) { return __fmaf_rn(b, b, -__fmul_rn(d, c)); }
+
 // ---------------------------------------------------------------- quadratic roots
 // Solve d t^2 + 2 b t + c = 0 choosing the form of each root that avoids cancellation.
 PHX_D void robust_roots(float& t1, float& t2, float& disc, float& sdisc, const float d, const float b, const float c)
 {
-    disc = b * b - d * c;
+    disc = fx_disc(d, b, c);
     sdisc = disc > 0.f ? sqrtf(disc) : 0.f;
     float q = b > 0.f ? -(b + sdisc) : -(b - sdisc);
     float root1 = q / d;
@@ -118,7 +158,7 @@ PHX_D void robust_roots(float& t1, float& t2, float& disc, float& sdisc, const f
 }
 PHX_D void robust_roots_disq(const float t_min, float& t1, float& t2, float& disc, float& sdisc, const float d, const float b, const float c)
 {
-    disc = b * b - d * c;
+    disc = fx_disc(d, b, c);
     sdisc = disc > 0.f ? sqrtf(disc) : 0.f;
     float q = b > 0.f ? -(b + sdisc) : -(b - sdisc);
     float root1 = sdisc > 0.f ? q / d : t_min;
@@ -149,9 +189,9 @@ PHX_D bool leaf_sphere(float4& isect, const float4& q0, float t_min, const float
     float radius = q0.w;
     float3 O = o - center;
     float3 D = dir;
-    float b = dot(O, D);
-    float c = dot(O, O) - radius * radius;
-    float d = dot(D, D);
+    float b = fx_dot(O, D);
+    float c = __fmaf_rn(-radius, radius, fx_dot(O, O));
+    float d = fx_dot(D, D);
     float root1, root2, disc, sdisc;
     robust_roots(root1, root2, disc, sdisc, d, b, c);
     if (POLISH && sdisc > 0.f) {
@@ -164,9 +204,10 @@ PHX_D bool leaf_sphere(float4& isect, const float4& q0, float t_min, const float
     float t_cand = sdisc > 0.f ? (root1 > t_min ? root1 : root2) : t_min;
     bool valid = t_cand > t_min;
     if (valid) {
-        isect.x = (O.x + t_cand * D.x) / radius;
-        isect.y = (O.y + t_cand * D.y) / radius;
-        isect.z = (O.z + t_cand * D.z) / radius;
+        const float3 p = fx_at(O, t_cand, D);
+        isect.x = p.x / radius;
+        isect.y = p.y / radius;
+        isect.z = p.z / radius;
         isect.w = t_cand;
     }
     return valid;
@@ -179,12 +220,12 @@ PHX_D bool leaf_zsphere(float4& isect, const float4& q0, const float4& q1, float
     float3 O = o - center;
     float3 D = dir;
     const float radius = q0.w;
-    float b = dot(O, D);
-    float c = dot(O, O) - radius * radius;
+    float b = fx_dot(O, D);
+    float c = __fmaf_rn(-radius, radius, fx_dot(O, O));
     if (c > 0.f && b > 0.f) return false;   // outside and moving away
     const float zmax = center.z + q1.y;
     const float zmin = center.z + q1.x;
-    float d = dot(D, D);
+    float d = fx_dot(D, D);
     float t1sph, t2sph, disc, sdisc;
     robust_roots(t1sph, t2sph, disc, sdisc, d, b, c);
     if (POLISH && sdisc > 0.f) {
@@ -194,11 +235,11 @@ PHX_D bool leaf_zsphere(float4& isect, const float4& q0, const float4& q1, float
         double dd = (double)D.x * D.x + (double)D.y * D.y + (double)D.z * D.z;
         polish_roots(t1sph, t2sph, dd, bb, cc);
     }
-    float z1sph = o.z + t1sph * dir.z;
-    float z2sph = o.z + t2sph * dir.z;
+    float z1sph = __fmaf_rn(t1sph, dir.z, o.z);
+    float z2sph = __fmaf_rn(t2sph, dir.z, o.z);
     float idz = 1.f / dir.z;
-    float t_QCAP = (zmax - o.z) * idz;
-    float t_PCAP = (zmin - o.z) * idz;
+    float t_QCAP = __fmul_rn(zmax - o.z, idz);
+    float t_PCAP = __fmul_rn(zmin - o.z, idz);
     float t1cap = fminf(t_QCAP, t_PCAP);
     float t2cap = fmaxf(t_QCAP, t_PCAP);
     if (t1cap < t1sph || t1cap > t2sph) t1cap = t_min;
@@ -214,9 +255,10 @@ PHX_D bool leaf_zsphere(float4& isect, const float4& q0, const float4& q1, float
     if (valid) {
         isect.w = t_cand;
         if (t_cand == t1sph || t_cand == t2sph) {
-            isect.x = (O.x + t_cand * D.x) / radius;
-            isect.y = (O.y + t_cand * D.y) / radius;
-            isect.z = (O.z + t_cand * D.z) / radius;
+            const float3 p = fx_at(O, t_cand, D);
+            isect.x = p.x / radius;
+            isect.y = p.y / radius;
+            isect.z = p.z / radius;
         } else {
             isect.x = 0.f;
             isect.y = 0.f;
@@ -234,10 +276,10 @@ PHX_D bool leaf_cylinder(float4& isect, const float4& q0, const float4& q1, floa
     const float z2 = q1.y;
     const float ox = o.x, oy = o.y, oz = o.z;
     const float vx = dir.x, vy = dir.y, vz = dir.z;
-    const float r2 = r * r;
-    const float a = vx * vx + vy * vy;
-    const float b = ox * vx + oy * vy;
-    const float c = ox * ox + oy * oy - r2;
+    const float r2 = __fmul_rn(r, r);
+    const float a = fx_dot2(vx, vy, vx, vy);
+    const float b = fx_dot2(ox, oy, vx, vy);
+    const float c = __fsub_rn(fx_dot2(ox, oy, ox, oy), r2);
     float t_near, t_far, disc, sdisc;
     robust_roots_disq(t_min, t_near, t_far, disc, sdisc, a, b, c);
     if (POLISH && sdisc > 0.f) {
@@ -246,12 +288,14 @@ PHX_D bool leaf_cylinder(float4& isect, const float4& q0, const float4& q1, floa
         double cc = (double)ox * ox + (double)oy * oy - (double)r * r;
         polish_roots(t_near, t_far, aa, bb, cc);
     }
-    float z_near = oz + t_near * vz;
-    float z_far = oz + t_far * vz;
+    float z_near = __fmaf_rn(t_near, vz, oz);
+    float z_far = __fmaf_rn(t_far, vz, oz);
     const float t_z1cap = (z1 - oz) / vz;
-    const float r2_z1cap = (ox + t_z1cap * vx) * (ox + t_z1cap * vx) + (oy + t_z1cap * vy) * (oy + t_z1cap * vy);
+    const float x1 = __fmaf_rn(t_z1cap, vx, ox), y1 = __fmaf_rn(t_z1cap, vy, oy);
+    const float r2_z1cap = fx_dot2(x1, y1, x1, y1);
     const float t_z2cap = (z2 - oz) / vz;
-    const float r2_z2cap = (ox + t_z2cap * vx) * (ox + t_z2cap * vx) + (oy + t_z2cap * vy) * (oy + t_z2cap * vy);
+    const float x2 = __fmaf_rn(t_z2cap, vx, ox), y2 = __fmaf_rn(t_z2cap, vy, oy);
+    const float r2_z2cap = fx_dot2(x2, y2, x2, y2);
     const float INF = __int_as_float(0x7f800000);
     float t_cand = INF;
     if (t_near > t_min && z_near > z1 && z_near < z2 && t_near < t_cand) t_cand = t_near;
@@ -261,8 +305,8 @@ PHX_D bool leaf_cylinder(float4& isect, const float4& q0, const float4& q1, floa
     bool valid = t_cand > t_min && t_cand < INF;
     if (valid) {
         bool sheet = (t_cand == t_near || t_cand == t_far);
-        isect.x = sheet ? (ox + t_cand * vx) / r : 0.f;
-        isect.y = sheet ? (oy + t_cand * vy) / r : 0.f;
+        isect.x = sheet ? __fmaf_rn(t_cand, vx, ox) / r : 0.f;
+        isect.y = sheet ? __fmaf_rn(t_cand, vy, oy) / r : 0.f;
         isect.z = sheet ? 0.f : (t_cand == t_z1cap ? -1.f : 1.f);
         isect.w = t_cand;
     }
@@ -685,13 +729,13 @@ PHX_COLD float4 leaf_disc(const float4 q0, const float4 q1, const float t_min, c
         t4[0] = __ldg(src + 0); t4[1] = __ldg(src + 1); t4[2] = __ldg(src + 2); t4[3] = __ldg(src + 3); \
         q = t4;                                                                                  \
     }                                                                                            \
-    float3 origin = q ? xform_row(q, ray_o, 1.f) : ray_o;                                        \
-    float3 direction = q ? xform_row(q, ray_d, 0.f) : ray_d;                                     \
+    float3 origin = q ? fx_point(q, ray_o) : ray_o;                                              \
+    float3 direction = q ? fx_dir(q, ray_d) : ray_d;                                             \
     bool valid = false;
 
 #define PHX_LEAF_EPILOGUE                                                                        \
     if (valid && q) {                                                                            \
-        float3 n = xform_col(q, make_float3(isect.x, isect.y, isect.z), 0.f);                    \
+        float3 n = fx_normal(q, make_float3(isect.x, isect.y, isect.z));                         \
         isect.x = n.x; isect.y = n.y; isect.z = n.z;                                             \
     }                                                                                            \
     if (complement) {                                                                            \
@@ -715,6 +759,19 @@ PHX_LEAFFN float4 leaf_eval(const float4* __restrict__ node, const float4* __res
         case PHX_CSG_TORUS:    isect = leaf_torus(q0, t_min, origin, direction); valid = isect.w > t_min; break;
         default: break;
     }
+    PHX_LEAF_EPILOGUE
+}
+
+// the sphere, zsphere and cylinder leaves inlined into the caller (closest-hit kernels): no call, so
+// the caller's ray and traversal state need not survive one
+template <bool POLISH>
+PHX_D float4 leaf_fast(const float4* __restrict__ node, const float4* __restrict__ itra, const int ni, const float t_min,
+                       const float3& ray_o, const float3& ray_d)
+{
+    PHX_LEAF_PROLOGUE
+    if (typecode == PHX_CSG_ZSPHERE) valid = leaf_zsphere<POLISH>(isect, q0, q1, t_min, origin, direction);
+    else if (typecode == PHX_CSG_CYLINDER) valid = leaf_cylinder<POLISH>(isect, q0, q1, t_min, origin, direction);
+    else valid = leaf_sphere<POLISH>(isect, q0, t_min, origin, direction);
     PHX_LEAF_EPILOGUE
 }
 
@@ -944,6 +1001,40 @@ PHX_D bool intersect_tree3(float4& isect, const PhxCsgCtx& g, int root, unsigned
     return false;
 }
 
+// The same for two leaf_fast leaves, known on the host.  One loop body evaluates a leaf (left, right,
+// then whichever has to be looked at again), so the leaf code is inlined once.
+template <bool POLISH>
+PHX_D float4 intersect_tree3_fast(const float4* __restrict__ node, const float4* __restrict__ itra, int root, unsigned op, float t_min,
+                                  const float3& o, const float3& d, unsigned& err)
+{
+    float4 L = make_float4(0.f, 0.f, 0.f, 0.f), R = L;
+    int which = 1;                  // node evaluated in this turn: root + which
+    float t0 = t_min;
+    for (int it = 0; it < PHX_TREE3_LOOP_CAP + 1; it++) {
+        const float4 v = leaf_fast<POLISH>(node, itra, root + which, t0, o, d);
+        if (which == 1) L = v; else R = v;
+        if (it == 0) { which = 2; continue; }
+        int l_state = phx_classify(L, d, t_min);
+        int r_state = phx_classify(R, d, t_min);
+        bool leftIsCloser = fabsf(L.w) <= fabsf(R.w);
+        const bool l_promote = l_state == PHX_STATE_MISS && (signbit(L.x) || signbit(L.y));
+        const bool r_promote = r_state == PHX_STATE_MISS && (signbit(R.x) || signbit(R.y));
+        if (r_promote) { r_state = PHX_STATE_EXIT; leftIsCloser = true; }
+        if (l_promote) { l_state = PHX_STATE_EXIT; leftIsCloser = false; }
+        const int ctrl = phx_csg_lookup((int)op, l_state, r_state, leftIsCloser);
+        if (ctrl < PHX_CTRL_LOOP_A) {
+            float4 result = ctrl == PHX_CTRL_RETURN_MISS ? make_float4(0.f, 0.f, 0.f, 0.f) : (ctrl == PHX_CTRL_RETURN_A ? L : R);
+            if (ctrl == PHX_CTRL_RETURN_FLIP_B) { result.x = -result.x; result.y = -result.y; result.z = -result.z; }
+            result.w = copysignf(result.w, 1.f);
+            return result;
+        }
+        which = ctrl == PHX_CTRL_LOOP_A ? 1 : 2;
+        t0 = fabsf(which == 1 ? L.w : R.w) + PHX_CSG_PROPAGATE_EPSILON;
+    }
+    err |= PHX_STATUS_CSG_STACK;
+    return make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // ---------------------------------------------------------------- tree
 template <int CV>
 PHX_D bool intersect_tree(float4& isect, const PhxCsgCtx& g, int root, float t_min, const float3& o, const float3& d, unsigned& err)
@@ -1060,4 +1151,18 @@ PHX_D bool intersect_prim(float4& isect, const PhxCsgCtx& g, int root, float t_m
     if (typecode < PHX_CSG_NODE) return intersect_tree<CV>(isect, g, root, t_min, o, d, err);
     if constexpr (PHX_CV_F(CV)) return intersect_list<CV>(isect, g, root, root, typecode, t_min, o, d, err);
     return false;
+}
+
+// Any prim, out of line: the closest-hit kernels call it for the leaves whose kind (PHX_KIND_*) is not
+// inlined there.
+struct PhxPrimHit { float4 is; unsigned status; bool valid; };
+template <int CV>
+PHX_COLD PhxPrimHit intersect_prim_any(const float4* __restrict__ node, const float4* __restrict__ itra, const float4* __restrict__ plan,
+                                       const int root, const float t_min, const float3 o, const float3 d)
+{
+    const PhxCsgCtx g = { node, itra, plan };
+    PhxPrimHit h;
+    h.status = 0u;
+    h.valid = intersect_prim<CV>(h.is, g, root, t_min, o, d, h.status);
+    return h;
 }

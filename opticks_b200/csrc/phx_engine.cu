@@ -95,8 +95,10 @@ struct phx_engine {
     DevBuf<float4> node, itra, plan, inst_inv;
     PhxCsgCtx csg = { nullptr, nullptr, nullptr };
     DevBuf<phx_bvh4_node> bvh;
-    DevBuf<phx_leaf> leaves, globals;
-    DevBuf<float4> leaf_sph, global_sph;   // world bounding sphere per leaf (centre, radius)
+    DevBuf<phx_leaf> leaves;               // the global leaves, then the hierarchy's
+    DevBuf<float4> leaf_sph;               // world bounding sphere per leaf (centre, radius)
+    DevBuf<float4> global_q;               // plain global leaves (PhxScene.global_q)
+    unsigned kind_mask = 0u;
     int num_global = 0;
     float cull[4] = { 0.f, 0.f, 0.f, 0.f };
     int num_node = 0, num_prim = 0, num_inst = 0, num_leaf = 0, bvh_depth = 0;
@@ -168,11 +170,10 @@ static PhxScene scene_of(const phx_engine* e, int polish)
     S.inst_inv = e->inst_inv.p;
     S.csg = e->csg;
     (void)polish;
-    S.globals = e->globals.p;
     S.leaf_sph = e->leaf_sph.p;
-    S.global_sph = e->global_sph.p;
+    S.global_q = e->global_q.p;
     S.num_global = e->num_global;
-    S.num_leaf = e->num_leaf;
+    S.kind_mask = e->kind_mask;
     S.cull = make_float4(e->cull[0], e->cull[1], e->cull[2], e->cull[3]);
     S.bvh_empty = e->num_leaf == 0;
     S.empty = e->num_leaf == 0 && e->num_global == 0;
@@ -651,6 +652,19 @@ static const char* check_prim_nodes(const phx_geometry* geo, int root)
     return nullptr;
 }
 
+// the kind of a prim (PHX_KIND_*): what the closest-hit kernels can evaluate inline
+static uint32_t prim_kind(const phx_geometry* geo, int root)
+{
+    auto typecode = [&](int ni) { uint32_t tc; memcpy(&tc, geo->node + 16 * (size_t)ni + 14, 4); return tc; };
+    auto simple = [](uint32_t tc) { return tc == PHX_CSG_SPHERE || tc == PHX_CSG_ZSPHERE || tc == PHX_CSG_CYLINDER; };
+    const uint32_t tc = typecode(root);
+    if (simple(tc)) return PHX_KIND_LEAF;
+    if (tc < PHX_CSG_UNION || tc > PHX_CSG_DIFFERENCE) return PHX_KIND_ANY;
+    uint32_t num;
+    memcpy(&num, geo->node + 16 * (size_t)root, 4);       // subNum, checked against the table before
+    return num == 3u && simple(typecode(root + 1)) && simple(typecode(root + 2)) ? PHX_KIND_TREE3 + tc - PHX_CSG_UNION : PHX_KIND_ANY;
+}
+
 // prim-frame sphere: the smaller of the box sphere and the tree sphere
 static PhxSph prim_sphere(const phx_geometry* geo, int p)
 {
@@ -965,7 +979,7 @@ int phx_destroy(phx_engine* e)
     if (e->planck_tex) cudaDestroyTextureObject(e->planck_tex);
     if (e->planck_arr) cudaFreeArray(e->planck_arr);
     e->node.release(); e->itra.release(); e->plan.release(); e->inst_inv.release(); e->prim_node_d.release();
-    e->bvh.release(); e->leaves.release(); e->globals.release(); e->leaf_sph.release(); e->global_sph.release(); e->optical.release(); e->rng.release();
+    e->bvh.release(); e->leaves.release(); e->leaf_sph.release(); e->global_q.release(); e->optical.release(); e->rng.release();
     e->gs.release(); e->gs_off.release(); e->gs_event.release(); e->photon.release(); e->seq.release();
     e->hit.release(); e->hitword.release(); e->wordoff.release(); e->blocksum.release(); e->sensor.release();
     e->counters.release(); e->status.release(); e->ev_start.release(); e->ev_left.release();
@@ -1125,16 +1139,39 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     if (3 * (bv.max_depth + 1) + 4 > PHX_BVH_STACK) { phx_destroy(e); return phx_fail(-1, "phx_create: BVH depth %d exceeds traversal stack", bv.max_depth); }
     PHX_TRYCU(e->bvh.ensure(std::max<size_t>(1, bv.nodes.size())));
     if (!bv.nodes.empty()) PHX_TRYCU(cudaMemcpy(e->bvh.p, bv.nodes.data(), bv.nodes.size() * sizeof(phx_bvh4_node), cudaMemcpyHostToDevice));
-    PHX_TRYCU(e->leaves.ensure(std::max<size_t>(1, bv.leaves.size())));
-    if (!bv.leaves.empty()) PHX_TRYCU(cudaMemcpy(e->leaves.p, bv.leaves.data(), bv.leaves.size() * sizeof(phx_leaf), cudaMemcpyHostToDevice));
-    PHX_TRYCU(e->leaf_sph.ensure(std::max<size_t>(1, bv.leaf_sphere.size() / 4)));
-    if (!bv.leaf_sphere.empty()) PHX_TRYCU(cudaMemcpy(e->leaf_sph.p, bv.leaf_sphere.data(), bv.leaf_sphere.size() * sizeof(float), cudaMemcpyHostToDevice));
-    PHX_TRYCU(e->global_sph.ensure(std::max<size_t>(1, bv.global_sphere.size() / 4)));
-    if (!bv.global_sphere.empty()) PHX_TRYCU(cudaMemcpy(e->global_sph.p, bv.global_sphere.data(), bv.global_sphere.size() * sizeof(float), cudaMemcpyHostToDevice));
     e->num_global = (int)bv.globals.size();
     memcpy(e->cull, bv.cull, sizeof(e->cull));
-    PHX_TRYCU(e->globals.ensure(std::max<size_t>(1, bv.globals.size())));
-    if (!bv.globals.empty()) PHX_TRYCU(cudaMemcpy(e->globals.p, bv.globals.data(), bv.globals.size() * sizeof(phx_leaf), cudaMemcpyHostToDevice));
+    {
+        // global leaves first, then the hierarchy's, each with its prim's kind in the root's upper bits
+        // (left out of a node table that needs those bits)
+        std::vector<phx_leaf> all = bv.globals;
+        all.insert(all.end(), bv.leaves.begin(), bv.leaves.end());
+        std::vector<float> sph = bv.global_sphere;
+        sph.insert(sph.end(), bv.leaf_sphere.begin(), bv.leaf_sphere.end());
+        std::vector<float> gq(std::max<size_t>(1, bv.globals.size()) * 8, 0.f);
+        for (size_t g = 0; g < bv.globals.size(); g++) {
+            const float* q = geo->node + 16 * (size_t)all[g].node_offset;
+            const float* m = &inv[16 * (size_t)all[g].inst];
+            uint32_t tc, tw;
+            memcpy(&tc, q + 14, 4);
+            memcpy(&tw, q + 15, 4);
+            bool plain = tw == 0u && (tc == PHX_CSG_SPHERE || tc == PHX_CSG_BOX3);
+            for (int k = 0; k < 16; k++) plain = plain && m[k] == (k % 5 == 0 ? 1.f : 0.f);
+            if (!plain) continue;
+            memcpy(&gq[8 * g], q, 16);
+            memcpy(&gq[8 * g + 4], &tc, 4);
+        }
+        if (geo->num_node < (1 << PHX_LEAF_KIND)) {
+            e->kind_mask = 7u << PHX_LEAF_KIND;
+            for (phx_leaf& L : all) L.node_offset |= (int32_t)(prim_kind(geo, L.node_offset) << PHX_LEAF_KIND);
+        }
+        PHX_TRYCU(e->leaves.ensure(std::max<size_t>(1, all.size())));
+        if (!all.empty()) PHX_TRYCU(cudaMemcpy(e->leaves.p, all.data(), all.size() * sizeof(phx_leaf), cudaMemcpyHostToDevice));
+        PHX_TRYCU(e->leaf_sph.ensure(std::max<size_t>(1, sph.size() / 4)));
+        if (!sph.empty()) PHX_TRYCU(cudaMemcpy(e->leaf_sph.p, sph.data(), sph.size() * sizeof(float), cudaMemcpyHostToDevice));
+        PHX_TRYCU(e->global_q.ensure(gq.size() / 4));
+        PHX_TRYCU(cudaMemcpy(e->global_q.p, gq.data(), gq.size() * sizeof(float), cudaMemcpyHostToDevice));
+    }
     PHX_TRYCU(e->inst_inv.ensure(inv.size() / 4));
     PHX_TRYCU(cudaMemcpy(e->inst_inv.p, inv.data(), inv.size() * sizeof(float), cudaMemcpyHostToDevice));
 

@@ -7,11 +7,6 @@
 #include "phx_physics.cuh"
 
 #define PHX_BVH_STACK 48
-// phx_visit_node orders the hit children with a sorting network on integer keys (0: insertion
-// sort on the distances)
-#ifndef PHX_VISIT_SORTNET
-#define PHX_VISIT_SORTNET 1
-#endif
 // leaf steps are taken when leaf-ready lanes x this weight >= node-ready lanes (or no node work is left)
 #ifndef PHX_TRACE_LEAF_WEIGHT
 #define PHX_TRACE_LEAF_WEIGHT 1
@@ -19,28 +14,26 @@
 
 struct PhxScene {
     const phx_bvh4_node* bvh;   // root at 0
-    const phx_leaf* leaves;
-    const phx_leaf* globals;    // leaves tested first by every ray (boxes spanning much of the scene)
-    const float4* leaf_sph;     // world bounding sphere (centre, radius) of each hierarchy leaf
-    const float4* global_sph;   // and of each global leaf
+    const phx_leaf* leaves;     // the global leaves (tested first by every ray: boxes spanning much of the
+                                // scene), then the hierarchy's
+    const float4* leaf_sph;     // world bounding sphere (centre, radius) of each
+    const float4* global_q;     // two rows per global leaf: parameters of a plain leaf under the identity
+                                // instance, and its typecode (word 0; 0: any other leaf)
     const float4* inst_inv;     // (num_inst*4) rows of the world->object 4x4 (row-vector convention)
     PhxCsgCtx csg;
     float4 cull;                // ball no hierarchy leaf reaches: centre xyz, radius^2 (0: none)
     int num_global;
-    int num_leaf;               // hierarchy leaves (stack ranges from here on address the global leaves)
+    unsigned kind_mask;         // bits of phx_leaf.node_offset that hold the leaf's kind (PHX_LEAF_KIND)
     int bvh_empty;              // no hierarchy leaves
     int empty;                  // no leaves at all
 };
 
 struct PhxBest {
     float t;
-    int4 L;                     // leaf (inst, node_offset, gp_bd, ii_id); L.x < 0 : none
-    float4 isect;
-    float lposcost;
+    int leaf;                   // index into the scene's leaves; < 0 : none
+    float3 n;                   // object-frame normal
 };
 
-// IS program of CSGOptiX/CSGOptiX7.cu:896-967 for one (instance, prim) leaf: object-frame
-// intersect_prim, keep the closest hit and its lposcost
 // Can the ray segment (tmin, tmax) meet the ball (centre, radius)?  The radius is padded on the
 // host beyond FP32 error, so a false answer never hides a hit of the leaf inside the ball.
 PHX_D bool phx_ball_overlaps(const float4 b, const float3& o, const float3& d, float tmin, float tmax)
@@ -54,67 +47,172 @@ PHX_D bool phx_ball_overlaps(const float4 b, const float3& o, const float3& d, f
     return tc + h >= tmin && tc - h <= tmax;
 }
 
+// IS program of CSGOptiX/CSGOptiX7.cu:896-967 for one (instance, prim) leaf: object-frame
+// intersect_prim, keep the closest hit.  `li` indexes the scene's leaves, L is that record.
+// The usual prims (PHX_KIND_LEAF, PHX_KIND_TREE3) are evaluated inline: the kind comes with the leaf,
+// so the chain of dependent node loads that finds it out and the calls per leaf go away.  Identity and
+// lposcost of the hit are looked up once a ray (phx_best_prd), not at every closer hit.  With the plain
+// global leaves below: 10M-photon detector event 13.15 -> 12.27 ms, 2^20 rays through the detector
+// 443 -> 402 us.
 template <int CV>
-PHX_D void phx_test_leaf(const PhxScene& S, const int4 L, const float4 ball, const float3& o, const float3& d, float tmin, PhxBest& B,
+PHX_D void phx_test_leaf(const PhxScene& S, const int li, const int4 L, const float3& o, const float3& d, float tmin, PhxBest& B,
                          unsigned& status)
 {
-    if (!phx_ball_overlaps(ball, o, d, tmin, B.t)) return;
     const float4* q = S.inst_inv + 4 * L.x;
-    float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
-    const float3 lo = xform_row(m, o, 1.f);
-    const float3 ld = xform_row(m, d, 0.f);
+    const float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
+    const float3 lo = fx_point(m, o);
+    const float3 ld = fx_dir(m, d);
+    const unsigned kind = ((unsigned)L.y & S.kind_mask) >> PHX_LEAF_KIND;
+    const int root = (int)((unsigned)L.y & ~S.kind_mask);
     float4 is;
-    const bool valid = intersect_prim<CV>(is, S.csg, L.y, tmin, lo, ld, status);
+    bool valid;
+    if (kind >= PHX_KIND_TREE3) {
+        is = intersect_tree3_fast<PHX_CV_P(CV)>(S.csg.node, S.csg.itra, root, kind - PHX_KIND_TREE3 + 1u, tmin, lo, ld, status);
+        valid = is.w > 0.f;
+    } else if (kind == PHX_KIND_LEAF) {
+        is = leaf_fast<PHX_CV_P(CV)>(S.csg.node, S.csg.itra, root, tmin, lo, ld);
+        valid = is.w > tmin;
+    } else {
+        const PhxPrimHit h = intersect_prim_any<CV>(S.csg.node, S.csg.itra, S.csg.plan, root, tmin, lo, ld);
+        is = h.is;
+        valid = h.valid;
+        status |= h.status;
+    }
     // OptiX's interval rule: a report outside [tmin, tmax] is ignored (a convexpolyhedron wholly
     // behind the ray reports valid with t = 0, CSG/csg_intersect_leaf_convexpolyhedron.h:85-101)
     if (valid && is.w >= tmin && is.w < B.t) {
         B.t = is.w;
-        B.L = L;
-        B.isect = is;
-        const float3 lpos = lo + is.w * ld;
-        B.lposcost = lpos.z / sqrtf(dot(lpos, lpos));
+        B.leaf = li;
+        B.n = make_float3(is.x, is.y, is.z);
     }
 }
 
-// Visit BVH4 node ni: slab-test its four children against [tmin, tmax] and push the hit ones
-// (inner nodes and leaf ranges) far-to-near, so that the nearest is taken next.
-PHX_D void phx_visit_node(const PhxScene& S, int ni, const float3& inv, const float3& oi, float tmin, float tmax, int2* stk,
-                          int& sp, unsigned& status)
+// the hierarchy leaves [first, first + count) (counted from the first hierarchy leaf)
+template <int CV>
+PHX_D void phx_test_range(const PhxScene& S, int first, int count, const float3& o, const float3& d, float tmin, PhxBest& B, unsigned& status)
 {
-    const float4* nf = reinterpret_cast<const float4*>(S.bvh + ni);
-    const float4 lx = __ldg(nf + 0), hx = __ldg(nf + 1), ly = __ldg(nf + 2), hy = __ldg(nf + 3);
-    const float4 lz = __ldg(nf + 4), hz = __ldg(nf + 5);
-    const int4 ch = __ldg(reinterpret_cast<const int4*>(nf + 6));
-    const float lxa[4] = { lx.x, lx.y, lx.z, lx.w }, hxa[4] = { hx.x, hx.y, hx.z, hx.w };
-    const float lya[4] = { ly.x, ly.y, ly.z, ly.w }, hya[4] = { hy.x, hy.y, hy.z, hy.w };
-    const float lza[4] = { lz.x, lz.y, lz.z, lz.w }, hza[4] = { hz.x, hz.y, hz.z, hz.w };
+    for (int li = S.num_global + first; li < S.num_global + first + count; li++) {
+        const int4 L = __ldg(reinterpret_cast<const int4*>(S.leaves + li));
+        if (phx_ball_overlaps(__ldg(S.leaf_sph + li), o, d, tmin, B.t)) phx_test_leaf<CV>(S, li, L, o, d, tmin, B, status);
+    }
+}
+
+// The global leaves, in order.  Plain spheres and boxes of the world solid (identity instance, no
+// node transform, no complement: the usual volumes around a detector) are solved from their parameter
+// row, without the instance transform, the node loads and the dispatch of the general leaf.
+template <int CV>
+PHX_D void phx_test_globals(const PhxScene& S, const float3& o, const float3& d, float tmin, PhxBest& B, unsigned& status)
+{
+    for (int g = 0; g < S.num_global; g++) {
+        const float4 q0 = __ldg(S.global_q + 2 * g);
+        const unsigned tc = __float_as_uint(__ldg(&S.global_q[2 * g + 1].x));
+        if (tc == PHX_CSG_SPHERE || tc == PHX_CSG_BOX3) {
+            float4 is;
+            bool valid;
+            if (tc == PHX_CSG_SPHERE) valid = leaf_sphere<PHX_CV_P(CV)>(is, q0, tmin, o, d);
+            else { is = leaf_box3(q0, tmin, o, d); valid = is.w > tmin; }
+            if (valid && is.w < B.t) {
+                B.t = is.w;
+                B.leaf = g;
+                B.n = make_float3(is.x, is.y, is.z);
+            }
+        } else {
+            const int4 L = __ldg(reinterpret_cast<const int4*>(S.leaves + g));
+            if (phx_ball_overlaps(__ldg(S.leaf_sph + g), o, d, tmin, B.t)) phx_test_leaf<CV>(S, g, L, o, d, tmin, B, status);
+        }
+    }
+}
+
+// A ray's slab constants: reciprocal direction and -origin/direction per axis, each as a pair of
+// equal floats (the operand form of the packed FP32 instructions), and the byte offset of the box
+// side the ray meets first in a node's (lo, hi) row pair of the axis.
+struct PhxSlabs {
+    unsigned long long ix, iy, iz, ox, oy, oz;
+    unsigned nx, ny, nz;
+};
+
+PHX_D unsigned long long phx_pair(float a, float b)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+PHX_D void phx_unpair(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+PHX_D unsigned long long phx_fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+PHX_D float phx_max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+PHX_D float phx_min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// zero direction components are nudged, so every reciprocal is finite
+PHX_D void phx_ray_slabs(const float3& o, const float3& d, PhxSlabs& R)
+{
+    const float3 dd = make_float3(fabsf(d.x) < 1e-30f ? copysignf(1e-30f, d.x) : d.x,
+                                  fabsf(d.y) < 1e-30f ? copysignf(1e-30f, d.y) : d.y,
+                                  fabsf(d.z) < 1e-30f ? copysignf(1e-30f, d.z) : d.z);
+    const float3 inv = make_float3(1.f / dd.x, 1.f / dd.y, 1.f / dd.z);
+    R.ix = phx_pair(inv.x, inv.x); R.iy = phx_pair(inv.y, inv.y); R.iz = phx_pair(inv.z, inv.z);
+    const float3 oi = make_float3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
+    R.ox = phx_pair(oi.x, oi.x); R.oy = phx_pair(oi.y, oi.y); R.oz = phx_pair(oi.z, oi.z);
+    R.nx = (__float_as_uint(inv.x) >> 31) << 4;
+    R.ny = (__float_as_uint(inv.y) >> 31) << 4;
+    R.nz = (__float_as_uint(inv.z) >> 31) << 4;
+}
+
+// Visit BVH4 node ni: slab-test its four children against [tmin, tmax] and push the hit ones
+// (inner nodes and leaf ranges) far-to-near, so that the nearest is taken next.  A visit is bound by
+// issue and by its L1 loads (12 a ray on the detector's water rays), so it is kept short: the near and
+// far side of each axis are chosen by address instead of by min and max, two children share each
+// multiply-add (packed FP32), three-input min and max close the interval, and the pushed distance is the
+// sort key itself.  10M-photon detector event 13.77 -> 13.15 ms against four unpacked slab tests.
+PHX_D void phx_visit_node(const PhxScene& S, int ni, const PhxSlabs& R, float tmin, float tmax, int2* stk, int& sp, unsigned& status)
+{
+    const char* nb = reinterpret_cast<const char*>(S.bvh);
+    const unsigned at = (unsigned)ni << 7;
+    const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + R.nx)));
+    const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + (R.nx ^ 16u))));
+    const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 32u + R.ny)));
+    const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 32u + (R.ny ^ 16u))));
+    const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 64u + R.nz)));
+    const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 64u + (R.nz ^ 16u))));
+    const int4 ch = __ldg(reinterpret_cast<const int4*>(nb + (at + 96u)));
     const int cha[4] = { ch.x, ch.y, ch.z, ch.w };
-    float tn[4];
-    int hitmask = 0;
+    unsigned key[4];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const float tx0 = fmaf(lxa[c], inv.x, oi.x), tx1 = fmaf(hxa[c], inv.x, oi.x);
-        const float ty0 = fmaf(lya[c], inv.y, oi.y), ty1 = fmaf(hya[c], inv.y, oi.y);
-        const float tz0 = fmaf(lza[c], inv.z, oi.z), tz1 = fmaf(hza[c], inv.z, oi.z);
-        const float tnear = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
-        const float tfar = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tmax));
-        // slab arithmetic slack: boxes are padded on the host, and a relative slack here
-        tn[c] = tnear;
-        if (cha[c] != 0 && tnear <= tfar * 1.00001f + 1e-4f) hitmask |= 1 << c;
-    }
-#if PHX_VISIT_SORTNET
-    // order by a 4-key sorting network: key = the near distance's magnitude bits with the child
-    // slot in the two low bits, all ones for a missed child (sorts last).  For tnear >= 0 the bits
-    // order like the floats; the pushed distance itself is the exact tnear.
-    unsigned k0, k1, k2, k3;
-    {
-        unsigned kk[4];
+    for (int h = 0; h < 2; h++) {
+        float x0[2], x1[2], y0[2], y1[2], z0[2], z1[2];
+        phx_unpair(phx_fma2(h ? nx.y : nx.x, R.ix, R.ox), x0[0], x0[1]);
+        phx_unpair(phx_fma2(h ? fx.y : fx.x, R.ix, R.ox), x1[0], x1[1]);
+        phx_unpair(phx_fma2(h ? ny.y : ny.x, R.iy, R.oy), y0[0], y0[1]);
+        phx_unpair(phx_fma2(h ? fy.y : fy.x, R.iy, R.oy), y1[0], y1[1]);
+        phx_unpair(phx_fma2(h ? nz.y : nz.x, R.iz, R.oz), z0[0], z0[1]);
+        phx_unpair(phx_fma2(h ? fz.y : fz.x, R.iz, R.oz), z1[0], z1[1]);
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            kk[c] = (hitmask >> c) & 1 ? ((__float_as_uint(tn[c]) & 0x7ffffffcu) | (unsigned)c) : 0xffffffffu;
-        k0 = kk[0]; k1 = kk[1]; k2 = kk[2]; k3 = kk[3];
+        for (int q = 0; q < 2; q++) {
+            const int c = 2 * h + q;
+            const float tnear = phx_max3(fmaxf(x0[q], y0[q]), z0[q], tmin);
+            const float tfar = phx_min3(fminf(x1[q], y1[q]), z1[q], tmax);
+            // slab arithmetic slack: boxes are padded on the host, and a relative slack here.
+            // key: the near distance's bits (not negative: they order like the floats) with the
+            // child slot in the two low bits, all ones for a missed child (sorts last)
+            const unsigned k = ((unsigned)max(__float_as_int(tnear), 0) & 0x7ffffffcu) | (unsigned)c;
+            key[c] = cha[c] != 0 && tnear <= fmaf(tfar, 1.00001f, 1e-4f) ? k : 0xffffffffu;
+        }
     }
-    unsigned t;
+    unsigned k0 = key[0], k1 = key[1], k2 = key[2], k3 = key[3], t;
     t = min(k0, k1); k1 = max(k0, k1); k0 = t;
     t = min(k2, k3); k3 = max(k2, k3); k2 = t;
     t = min(k0, k2); k2 = max(k0, k2); k0 = t;
@@ -123,41 +221,15 @@ PHX_D void phx_visit_node(const PhxScene& S, int ni, const float3& inv, const fl
     const unsigned ks[4] = { k0, k1, k2, k3 };
 #pragma unroll
     for (int j = 3; j >= 0; j--) {
-        const unsigned key = ks[j];
-        if (key == 0xffffffffu) continue;
+        const unsigned k = ks[j];
+        if (k == 0xffffffffu) continue;
         if (sp >= PHX_BVH_STACK) { status |= PHX_STATUS_BVH_STACK; continue; }
-        const unsigned c = key & 3u;
-        stk[sp] = make_int2(c == 0u ? cha[0] : c == 1u ? cha[1] : c == 2u ? cha[2] : cha[3],
-                            __float_as_int(c == 0u ? tn[0] : c == 1u ? tn[1] : c == 2u ? tn[2] : tn[3]));
+        // the pushed distance is the key's, at most a few ulp below the near distance (tmin bounds
+        // it where that is negative), so that no entry is dropped too early
+        const int child = k & 2u ? (k & 1u ? cha[3] : cha[2]) : (k & 1u ? cha[1] : cha[0]);
+        stk[sp] = make_int2(child, k < 4u ? __float_as_int(tmin) : (int)(k & ~3u));
         sp++;
     }
-#else
-    int order[4] = { 0, 1, 2, 3 };
-#pragma unroll
-    for (int i = 1; i < 4; i++)
-#pragma unroll
-        for (int j = i; j > 0; j--) {
-            if (tn[order[j]] < tn[order[j - 1]]) { int t = order[j]; order[j] = order[j - 1]; order[j - 1] = t; }
-        }
-#pragma unroll
-    for (int k = 3; k >= 0; k--) {
-        const int c = order[k];
-        if (!(hitmask & (1 << c))) continue;
-        if (sp >= PHX_BVH_STACK) { status |= PHX_STATUS_BVH_STACK; continue; }
-        stk[sp] = make_int2(cha[c], __float_as_int(tn[c])); sp++;
-    }
-#endif
-}
-
-// ray set-up shared by both traversal loops: reciprocal direction (zero components nudged) and
-// the slab offsets
-PHX_D void phx_ray_slabs(const float3& o, const float3& d, float3& inv, float3& oi)
-{
-    const float3 dd = make_float3(fabsf(d.x) < 1e-30f ? copysignf(1e-30f, d.x) : d.x,
-                                  fabsf(d.y) < 1e-30f ? copysignf(1e-30f, d.y) : d.y,
-                                  fabsf(d.z) < 1e-30f ? copysignf(1e-30f, d.z) : d.z);
-    inv = make_float3(1.f / dd.x, 1.f / dd.y, 1.f / dd.z);
-    oi = make_float3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
 }
 
 // The segment [tmin, t] lies inside the ball no hierarchy leaf reaches: skip the hierarchy.
@@ -170,10 +242,10 @@ PHX_D bool phx_culled(const PhxScene& S, const float3& o, const float3& d, float
     return dot(p0, p0) < S.cull.w && dot(p1, p1) < S.cull.w;
 }
 
-// PRD of a closest hit (CH program CSGOptiX/CSGOptiX7.cu:776-874), or of a miss
-PHX_D void phx_best_prd(const PhxScene& S, const PhxBest& B, PhxPRD& prd)
+// PRD of a closest hit (CH program CSGOptiX/CSGOptiX7.cu:776-874, lposcost of the IS program), or of a miss
+PHX_D void phx_best_prd(const PhxScene& S, const PhxBest& B, const float3& o, const float3& d, PhxPRD& prd)
 {
-    if (B.L.x < 0) {
+    if (B.leaf < 0) {
         prd.gp_bd = 0xffffffffu;
         prd.ii_id = 0xffffffffu;
         prd.normal = make_float3(0.f, 0.f, 0.f);
@@ -181,13 +253,15 @@ PHX_D void phx_best_prd(const PhxScene& S, const PhxBest& B, PhxPRD& prd)
         prd.lposcost = 0.f;
         return;
     }
-    const float4* q = S.inst_inv + 4 * B.L.x;
-    float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
-    prd.normal = xform_col(m, make_float3(B.isect.x, B.isect.y, B.isect.z), 0.f);
+    const int4 L = __ldg(reinterpret_cast<const int4*>(S.leaves + B.leaf));
+    const float4* q = S.inst_inv + 4 * L.x;
+    const float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
+    prd.normal = fx_normal(m, B.n);
     prd.distance = B.t;
-    prd.lposcost = B.lposcost;
-    prd.gp_bd = (unsigned)B.L.z;
-    prd.ii_id = (unsigned)B.L.w;
+    const float3 lpos = fx_at(fx_point(m, o), B.t, fx_dir(m, d));
+    prd.lposcost = lpos.z / sqrtf(fx_mix(lpos.x, lpos.x, lpos.y, lpos.y, lpos.z, lpos.z));
+    prd.gp_bd = (unsigned)L.z;
+    prd.ii_id = (unsigned)L.w;
 }
 
 // Closest hit over all (instance, prim) leaves: restates optixTrace over the IAS with the
@@ -207,46 +281,41 @@ PHX_D bool phx_trace(const PhxScene& S, const float3& o, const float3& d, float 
     if (S.empty) return false;
     PhxBest B;
     B.t = tmax;
-    B.L = make_int4(-1, 0, 0, 0);
-    B.isect = make_float4(0.f, 0.f, 0.f, 0.f);
-    B.lposcost = 0.f;
-    for (int g = 0; g < S.num_global; g++)
-        phx_test_leaf<CV>(S, __ldg(reinterpret_cast<const int4*>(S.globals + g)), __ldg(S.global_sph + g), o, d, tmin, B, status);
+    B.leaf = -1;
+    B.n = make_float3(0.f, 0.f, 0.f);
+    phx_test_globals<CV>(S, o, d, tmin, B, status);
     if (!S.bvh_empty && !phx_culled(S, o, d, tmin, B.t)) {
-        float3 inv, oi;
-        phx_ray_slabs(o, d, inv, oi);
+        PhxSlabs R;
+        phx_ray_slabs(o, d, R);
         int2 stk[PHX_BVH_STACK];     // node or leaf range, near distance bits
-        int sp = 0;
-        stk[sp] = make_int2(0, __float_as_int(tmin)); sp++;
+        int sp = 1;
+        stk[0] = make_int2(0, __float_as_int(tmin));
         // Each step the lanes of the warp that traverse together vote: either the lanes whose next
         // entry is an inner node visit it, or the lanes whose next entry is a leaf range test it.
         // Every lane still takes its own entries in its own near-first order; the vote only
         // gathers the expensive leaf tests into steps where many lanes run them.
         const unsigned mask = __activemask();
         for (;;) {
-            while (sp > 0 && __int_as_float(stk[sp - 1].y) > B.t) sp--;
-            const bool leaf_top = sp > 0 && stk[sp - 1].x < 0;
+            int2 top = make_int2(0, 0);
+            while (sp > 0 && __int_as_float((top = stk[sp - 1]).y) > B.t) sp--;
+            const bool leaf_top = sp > 0 && top.x < 0;
             const unsigned want_leaf = __ballot_sync(mask, leaf_top);
             const unsigned want_node = __ballot_sync(mask, sp > 0 && !leaf_top);
             if (!(want_leaf | want_node)) break;
             const bool leaf_step = want_node == 0u || __popc(want_leaf) * PHX_TRACE_LEAF_WEIGHT >= __popc(want_node);
             if (sp == 0 || leaf_top != leaf_step) continue;
             sp--;
-            const int ni = stk[sp].x;
+            const int ni = top.x;
             if (leaf_step) {
                 const int enc = -ni - 1;
-                const int first = enc >> 3;
-                const int count = (enc & 7) + 1;
-                for (int li = first; li < first + count; li++)
-                    phx_test_leaf<CV>(S, __ldg(reinterpret_cast<const int4*>(S.leaves + li)), __ldg(S.leaf_sph + li), o, d, tmin,
-                                          B, status);
+                phx_test_range<CV>(S, enc >> 3, (enc & 7) + 1, o, d, tmin, B, status);
                 continue;
             }
-            phx_visit_node(S, ni, inv, oi, tmin, B.t, stk, sp, status);
+            phx_visit_node(S, ni, R, tmin, B.t, stk, sp, status);
         }
     }
-    phx_best_prd(S, B, prd);
-    return B.L.x >= 0;
+    phx_best_prd(S, B, o, d, prd);
+    return B.leaf >= 0;
 }
 
 struct PhxLoopCfg {

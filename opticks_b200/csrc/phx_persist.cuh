@@ -154,6 +154,15 @@ PHX_STEPFN_P int phx_propagate_step(PhxPhoton& p, curandStateXORWOW& rng, PhxPRD
 }
 #endif
 
+// The adjoint's physics step out of line, for the loops that hold a path over many bounces: compiled
+// apart from the closest-hit search, its roundings are those of the wavefront's physics kernel (the
+// pathwise terms are differences of nearly equal hits, which any other rounding shows in).
+PHX_COLD int propagate_adj(PhxPhoton& p, curandStateXORWOW& rng, PhxPRD prd, const PhxProps& P, unsigned& status, PhxScore* sc)
+{
+    prd.normal = fx_unit(prd.normal);
+    return propagate<true>(p, rng, prd, P, status, sc);
+}
+
 struct PhxLane {
     PhxPhoton p;
     curandStateXORWOW rng;
@@ -293,8 +302,7 @@ PHX_D bool persist_step(PhxLane& L, const PersistArgs& A, unsigned& status, PhxS
     if (prd.boundary() == 0xffffu) return true;
     int command;
     if (ADJ) {
-        prd.normal = normalize(prd.normal);
-        command = propagate<ADJ>(L.p, L.rng, prd, A.P, status, sc);
+        command = propagate_adj(L.p, L.rng, prd, A.P, status, sc);
     } else {
         command = phx_propagate_step(L.p, L.rng, prd, A.P, status);
     }

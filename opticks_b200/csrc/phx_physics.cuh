@@ -841,20 +841,21 @@ PHX_D void adj_probe(PhxAdjSeg& seg, const PhxScore& sc, const PhxPhoton& p, con
     const float mag = length(sc.tpos) + D * length(sc.tdir);
     if (!(mag > 0.f) || !sc.prim_node) return;
     const float eps = PHX_ADJ_PROBE_SHIFT / mag;
-    const float3 o2 = p.pos + eps * sc.tpos;
-    const float3 d2 = normalize(p.mom + eps * sc.tdir);
+    const float3 o2 = fx_at(p.pos, eps, sc.tpos);
+    const float3 d2 = fx_unit_mix(fx_at(p.mom, eps, sc.tdir));
     const unsigned gp = prd.gp_bd >> 16, ii = prd.ii_id >> 16;
     const float4* q = sc.inst_inv + 4 * ii;
-    float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
-    const float3 lo = xform_row(m, o2, 1.f), ld = xform_row(m, d2, 0.f);
+    const float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
+    // the roundings of the closest-hit search: the differences below compare the two hits
+    const float3 lo = fx_point(m, o2), ld = fx_dir(m, d2);
     const float tmin = (p.obf & sc.eps0_mask) ? sc.tmin0 : sc.tmin;
     float4 is;
     unsigned st = 0;
     if (!intersect_prim<PHX_CV_FULL>(is, sc.csg, __ldg(sc.prim_node + gp), tmin, lo, ld, st)) return;
-    const float3 n2 = normalize(xform_col(m, make_float3(is.x, is.y, is.z), 0.f));
+    const float3 n2 = fx_unit_mix(fx_normal(m, make_float3(is.x, is.y, is.z)));
     if (dot(n1, n2) < 0.9f) return;
-    const float3 h1 = p.pos + D * p.mom;
-    const float3 h2 = o2 + is.w * d2;
+    const float3 h1 = fx_at(p.pos, D, p.mom);
+    const float3 h2 = fx_at(o2, is.w, d2);
     seg.dD = (is.w - D) / eps;
     seg.dpos_hit = (1.f / eps) * (h2 - h1);
     seg.dnormal = (1.f / eps) * (n2 - n1);

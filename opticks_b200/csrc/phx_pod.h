@@ -134,10 +134,17 @@ typedef struct {
 
 typedef struct { uint64_t seqhis[PHX_NSEQ]; uint64_t seqbnd[PHX_NSEQ]; } phx_seq;  // 32 B, sseq
 
+// Prim kinds the closest-hit kernels evaluate inline: a sphere, zsphere or cylinder leaf, or one operator
+// over two of them (PHX_KIND_TREE3 + operator - 1).  Any other prim is PHX_KIND_ANY.
+#define PHX_LEAF_KIND 28
+#define PHX_KIND_ANY 0u
+#define PHX_KIND_LEAF 1u
+#define PHX_KIND_TREE3 2u
+
 // BVH leaf record : one (instance, CSGPrim) pair
 typedef struct {
     int32_t  inst;          // index into the instance transform arrays
-    int32_t  node_offset;   // root node of the prim's CSG tree
+    int32_t  node_offset;   // root node of the prim's CSG tree, and its kind from bit PHX_LEAF_KIND on
     uint32_t gp_bd;         // (globalPrimIdx & 0xffff) << 16 | (boundary & 0xffff)
     uint32_t ii_id;         // (iindex & 0xffff) << 16 | (identity & 0xffff), identity = sensor_id+1
 } phx_leaf;

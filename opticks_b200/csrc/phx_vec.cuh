@@ -53,25 +53,6 @@ PHX_D float2 operator-(const float2& a, const float2& b) { return make_float2(a.
 PHX_D float dot2(const float2& a, const float2& b) { return a.x * b.x + a.y * b.y; }
 PHX_D float2 normalize2(const float2& v) { float invLen = 1.0f / sqrtf(dot2(v, v)); return make_float2(v.x * invLen, v.y * invLen); }
 
-// row-vector transform by a 4x4 stored as four float4 rows (q0..q3): v' = v * M (w = 1 point, 0 dir)
-PHX_D float3 xform_row(const float4* q, const float3& v, float w)
-{
-    float3 r;
-    r.x = q[0].x * v.x + q[1].x * v.y + q[2].x * v.z + q[3].x * w;
-    r.y = q[0].y * v.x + q[1].y * v.y + q[2].y * v.z + q[3].y * w;
-    r.z = q[0].z * v.x + q[1].z * v.y + q[2].z * v.z + q[3].z * w;
-    return r;
-}
-// column transform: v' = M * v using the upper 3x4 (used for normals with the inverse matrix)
-PHX_D float3 xform_col(const float4* q, const float3& v, float w)
-{
-    float3 r;
-    r.x = q[0].x * v.x + q[0].y * v.y + q[0].z * v.z + q[0].w * w;
-    r.y = q[1].x * v.x + q[1].y * v.y + q[1].z * v.z + q[1].w * w;
-    r.z = q[2].x * v.x + q[2].y * v.y + q[2].z * v.z + q[2].w * w;
-    return r;
-}
-
 // CLHEP Hep3Vector::rotateUz: rotate frame so that z goes along unit vector u.
 // Same float operation order as sysrap/smath.h:95-112 which restates CLHEP.
 PHX_D void rotate_uz(float3& d, const float3& u)

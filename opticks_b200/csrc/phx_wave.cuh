@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init
 
 // closest hit of every live path (CSGOptiX/CSGOptiX7.cu:477-490: tmin by the last flag, optixTrace)
 // resident 128-thread blocks per SM asked of the compiler for the closest-hit kernel (caps its
-// registers: 3 -> 168 registers, 12 warps per SM, no spills; 4 -> 128 with spills, measured slower)
+// registers: 3 -> 168 registers, 12 warps per SM; 4 -> 128 with spills, 12.7 ms against 12.3 for the
+// 10M-photon detector event)
 #ifndef PHX_WAVE_TRACE_MINB
 #define PHX_WAVE_TRACE_MINB 3
 #endif
@@ -391,10 +392,11 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
     bool drained = false;                 // the round's rays are all handed out
     bool has = false;                     // this lane holds a ray
     uint32_t s = 0u;
-    float3 o = make_float3(0.f, 0.f, 0.f), d = o, inv = o, oi = o;
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+    PhxSlabs R = {};
     float tmin = 0.f;
     PhxBest B;
-    B.t = 0.f; B.L = make_int4(-1, 0, 0, 0); B.isect = make_float4(0.f, 0.f, 0.f, 0.f); B.lposcost = 0.f;
+    B.t = 0.f; B.leaf = -1; B.n = o;
     int2 stk[PHX_BVH_STACK];         // node or leaf range, near distance bits
     int sp = 0;
     for (;;) {
@@ -420,13 +422,11 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
                 tmin = wave_tmin(W, q1);
                 o = make_float3(q0.x, q0.y, q0.z);
                 d = make_float3(q1.x, q1.y, q1.z);
-                phx_ray_slabs(o, d, inv, oi);
-                B.t = W.A.C.tmax; B.L = make_int4(-1, 0, 0, 0); B.isect = make_float4(0.f, 0.f, 0.f, 0.f); B.lposcost = 0.f;
+                phx_ray_slabs(o, d, R);
+                B.t = W.A.C.tmax; B.leaf = -1; B.n = make_float3(0.f, 0.f, 0.f);
                 sp = 0;
                 // the global leaves first, then the hierarchy unless the cull ball holds the segment
-                for (int g = 0; g < S.num_global; g++)
-                    phx_test_leaf<CV>(S, __ldg(reinterpret_cast<const int4*>(S.globals + g)), __ldg(S.global_sph + g), o, d, tmin, B,
-                                      status);
+                phx_test_globals<CV>(S, o, d, tmin, B, status);
                 if (!S.bvh_empty && !phx_culled(S, o, d, tmin, B.t)) { stk[0] = make_int2(0, __float_as_int(tmin)); sp = 1; }
                 has = true;
             }
@@ -434,17 +434,18 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
             idle = __ballot_sync(FULL, !has);
         }
         // finish the rays whose stacks are empty
+        int2 top = make_int2(0, 0);
         if (has) {
-            while (sp > 0 && __int_as_float(stk[sp - 1].y) > B.t) sp--;
+            while (sp > 0 && __int_as_float((top = stk[sp - 1]).y) > B.t) sp--;
             if (sp == 0) {
                 PhxPRD prd;
-                phx_best_prd(S, B, prd);
+                phx_best_prd(S, B, o, d, prd);
                 W.prd[s].nd = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
                 W.prd[s].lgi = make_uint4(__float_as_uint(prd.lposcost), prd.gp_bd, prd.ii_id, 0u);
                 has = false;
             }
         }
-        const bool leaf_top = has && stk[sp - 1].x < 0;
+        const bool leaf_top = has && top.x < 0;
         const unsigned want_leaf = __ballot_sync(FULL, leaf_top);
         const unsigned want_node = __ballot_sync(FULL, has && !leaf_top);
         if (!(want_leaf | want_node)) {
@@ -455,15 +456,12 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
         const bool leaf_step = want_node == 0u || __popc(want_leaf) * PHX_TRACE_LEAF_WEIGHT >= __popc(want_node);
         if (!has || leaf_top != leaf_step) continue;
         sp--;
-        const int ni = stk[sp].x;
+        const int ni = top.x;
         if (leaf_step) {
             const int enc = -ni - 1;
-            const int first = enc >> 3;
-            const int count = (enc & 7) + 1;
-            for (int li = first; li < first + count; li++)
-                phx_test_leaf<CV>(S, __ldg(reinterpret_cast<const int4*>(S.leaves + li)), __ldg(S.leaf_sph + li), o, d, tmin, B, status);
+            phx_test_range<CV>(S, enc >> 3, (enc & 7) + 1, o, d, tmin, B, status);
         } else {
-            phx_visit_node(S, ni, inv, oi, tmin, B.t, stk, sp, status);
+            phx_visit_node(S, ni, R, tmin, B.t, stk, sp, status);
         }
     }
     if (status) atomicOr(W.A.status, status);
@@ -475,8 +473,10 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
 // ends takes the next one of the list at once (one atomic per warp on the round's ray counter,
 // which the physics kernel left at zero), so the lanes of a warp do not wait for its longest path.
 // Photons, seq and hits are the same as the rounds would give.
+// (3 blocks of 128 per SM, 168 registers; with the closest-hit search inlined: 3 blocks 12.27 ms for the
+// 10M-photon detector event, 4 blocks 13.61, 5 blocks 13.36)
 template <int CV, bool ADJ = false>
-__global__ void __launch_bounds__(128) k_wave_tail(WaveArgs W)
+__global__ void __launch_bounds__(128, 3) k_wave_tail(WaveArgs W)
 {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
@@ -545,7 +545,7 @@ PHX_D bool wave_shade_path(const WaveArgs& W, const float4* st, uint32_t s, cons
     if (prd.boundary() != 0xffffu) {
         int command;
         if (ADJ) {
-            prd.normal = normalize(prd.normal);
+            prd.normal = fx_unit(prd.normal);
             command = propagate<true>(L.p, L.rng, prd, W.A.P, status, sc);
         } else {
             command = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
