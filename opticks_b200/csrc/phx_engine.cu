@@ -138,12 +138,12 @@ struct phx_engine {
     DevBuf<long long> counters;   // [0] num_hit, [1] queue head, [3] largest event
     DevBuf<long long> ev_start;
     DevBuf<unsigned> ev_left;
-    DevBuf<uint32_t> jump_pow, jump_tab;   // P_k = T^(skip 2^k) and per-call event jump matrices
-    DevBuf<uint32_t> jump4;                // 4-bit group tables of a single-event jump matrix
+    DevBuf<uint32_t> jump_digit;           // jump tables of every event digit (k_jump_digits)
+    DevBuf<uint32_t> jump4;                // a call's event jump tables (one, or one per genstep)
     DevBuf<uint32_t> ev_rng;               // per-call event-advanced XORWOW states (k_rng_event)
     cudaGraphExec_t batch_exec = nullptr;   // cached batched launch sequence (use_graph)
     PhxBatchCall batch_call;
-#define PHX_BATCH_BUFS 20
+#define PHX_BATCH_BUFS 19
     const void* batch_bufs[PHX_BATCH_BUFS] = {};
     unsigned long long batch_launch = 0;     // launch_key of the captured graph
     DevBuf<unsigned> status;
@@ -226,10 +226,10 @@ __global__ void k_rng_init(unsigned long long seed, unsigned long long offset, l
     rng[slots * 5 + slot] = s.v[4];
 }
 
-// exclusive scan of genstep photon counts (quad6 q0.w) into off[G+1] : replaces the
+// Exclusive scan, by one block of 1024 threads, of genstep photon counts (quad6 q0.w) into off[G+1] : replaces the
 // thrust reduce + iexpand seed buffer of qudarap/QEvt.cu:180-230 (photons find their genstep by
 // binary search over off, so no per-photon seed array is written or read)
-__global__ void k_genstep_offsets(const float4* gs, int G, long long* off)
+PHX_D void phx_genstep_offsets(const float4* gs, int G, long long* off)
 {
     __shared__ long long warp_tot[32];
     __shared__ long long carry;
@@ -259,6 +259,35 @@ __global__ void k_genstep_offsets(const float4* gs, int G, long long* off)
     if (threadIdx.x == 0) off[0] = 0;
 }
 
+__global__ void __launch_bounds__(1024) k_genstep_offsets(const float4* gs, int G, long long* off) { phx_genstep_offsets(gs, G, off); }
+
+// Everything a single-event call needs before its first photon, in one launch (each of these cost a
+// launch or a memset of its own, 2-4 us apiece, and the event's matrix 48 us): block 0 scans the
+// genstep counts and clears the call's counters, block 1 makes the event's jump tables, the others
+// clear the hit bits and the sensor counts.
+#define PHX_SETUP_WORDS 4096        // words a clearing block takes
+__global__ void __launch_bounds__(1024) k_call_setup(const float4* gs, int G, long long* off, unsigned long long event,
+                                                     const uint32_t* __restrict__ D, uint32_t* T, long long* counters, unsigned* status,
+                                                     uint32_t* hitword, long long nword, uint32_t* sensor, int num_sensor)
+{
+    __shared__ uint32_t col[PHX_JUMP_BITS * 5];
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < 2) counters[threadIdx.x] = 0;
+        if (threadIdx.x == 0) *status = 0u;
+        phx_genstep_offsets(gs, G, off);
+        return;
+    }
+    if (blockIdx.x == 1) {
+        if (event > 0ull) phx_event_table(event, D, T, col);
+        return;
+    }
+    const long long w0 = (long long)(blockIdx.x - 2) * PHX_SETUP_WORDS;
+    for (long long w = w0 + threadIdx.x; w < w0 + PHX_SETUP_WORDS; w += 1024) {
+        if (w < nword) hitword[w] = 0u;
+        else if (w - nword < (long long)num_sensor) sensor[w - nword] = 0u;
+    }
+}
+
 struct SimArgs {
     PhxScene S;
     PhxProps P;
@@ -272,8 +301,7 @@ struct SimArgs {
     unsigned long long skip;
     const uint32_t* rng;
     long long rng_slots;
-    const uint32_t* jump;      // event jump matrix (phx_rngjump.h) or null for cuRAND skipahead
-    const uint32_t* jump4;     // its 4-bit group tables, or null
+    const uint32_t* jump4;     // the event's jump tables (phx_event_table); unused for event 0
     phx_photon* photon;
     phx_seq* seq;
     uint32_t* hitword;
@@ -306,9 +334,7 @@ __global__ void __launch_bounds__(PHX_SIM_BLOCK, PHX_SIM_MINB) k_simulate(SimArg
             curand_init(0ull, (unsigned long long)photon_idx, 0ull, &rng);
         }
         if (a.event_index > 0ull) {
-            if (a.jump4) phx_rng_jump4(rng, a.jump4, a.skip * a.event_index);
-            else if (a.jump) phx_rng_jump(rng, a.jump, a.skip * a.event_index);
-            else skipahead(a.skip * a.event_index, &rng);
+            phx_rng_jump4(rng, a.jump4, a.skip * a.event_index);
         }
         PhxPhoton p;
         memset(&p, 0, sizeof(p));
@@ -983,7 +1009,7 @@ int phx_destroy(phx_engine* e)
     e->gs.release(); e->gs_off.release(); e->gs_event.release(); e->photon.release(); e->seq.release();
     e->hit.release(); e->hitword.release(); e->wordoff.release(); e->blocksum.release(); e->sensor.release();
     e->counters.release(); e->status.release(); e->ev_start.release(); e->ev_left.release();
-    e->jump_pow.release(); e->jump_tab.release(); e->jump4.release(); e->ev_rng.release();
+    e->jump_digit.release(); e->jump4.release(); e->ev_rng.release();
     e->merge.release();
     e->wslot.release(); e->wprd.release(); e->wsidx.release(); e->wact0.release(); e->wact1.release(); e->wfree.release(); e->wscore.release(); e->wcnt.release();
     e->wlive.release(); e->wlive_off.release(); e->wlive_blk.release(); e->wlive_tot.release();
@@ -1205,9 +1231,18 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     // ---- rng + small buffers
     {
         const std::vector<uint32_t> pw = phx_jump_powers(e->cfg.skipahead_event_offset);
-        PHX_TRYCU(e->jump_pow.ensure(pw.size()));
-        PHX_TRYCU(cudaMemcpy(e->jump_pow.p, pw.data(), pw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-        PHX_TRYCU(e->jump_tab.ensure(PHX_JUMP_MATW));
+        DevBuf<uint32_t> pow;
+        PHX_TRYCU(pow.ensure(pw.size()));
+        cudaError_t ce = cudaMemcpy(pow.p, pw.data(), pw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+        if (ce == cudaSuccess) ce = e->jump_digit.ensure((size_t)PHX_JUMP_DIGITS * 15 * PHX_JUMP_NIBW);
+        if (ce == cudaSuccess) {
+            k_jump_digits<<<PHX_JUMP_DIGITS * 15, PHX_JUMP_THREADS, 0, e->stream>>>(pow.p, e->jump_digit.p);
+            ce = cudaGetLastError();
+        }
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+        pow.release();
+        PHX_TRYCU(ce);
+        PHX_TRYCU(e->jump4.ensure(PHX_JUMP_NIBW));
     }
     PHX_TRYCU(e->status.ensure(4));
     PHX_TRYCU(e->counters.ensure(8));
@@ -1231,7 +1266,7 @@ static PersistArgs persist_args_from(const phx_engine* e, const SimArgs& a)
     A.gs = a.gs; A.gs_off = a.gs_off; A.G = a.G; A.N = a.N;
     A.photon_offset = a.photon_offset; A.event_index = a.event_index;
     A.gs_event = nullptr; A.ev_start = nullptr;
-    A.skip = a.skip; A.rng = a.rng; A.rng_slots = a.rng_slots; A.jump = a.jump; A.jump4 = a.jump4;
+    A.skip = a.skip; A.rng = a.rng; A.rng_slots = a.rng_slots; A.jump4 = a.jump4;
     A.photon = a.photon; A.seq = a.seq; A.hitword = a.hitword; A.hit_mask = a.hit_mask; A.status = a.status;
     A.regroup = 1; A.chunk = 1;
     return A;
@@ -1533,9 +1568,19 @@ struct PhxPlainBufs {
     uint32_t* blocksum;
     long long* counters;   // [0] num_hit, [1] queue head
     unsigned* status;
-    uint32_t* jump;        // one event jump matrix (PHX_JUMP_MATW words)
-    uint32_t* jump4;       // its 4-bit group tables (PHX_JUMP_NIBW words), or null to use the matrix
+    uint32_t* jump4;       // event jump tables (PHX_JUMP_NIBW words)
 };
+
+// k_call_setup on st (hitword and sensor may be null: nothing to clear)
+static void call_setup(const phx_engine* e, const float4* gs, int G, long long* gs_off, int event_index, uint32_t* jump4, long long* counters,
+                       unsigned* status, uint32_t* hitword, long long nword, uint32_t* sensor, cudaStream_t st)
+{
+    if (!hitword) nword = 0;
+    const int ns = sensor ? std::max(0, e->cfg.num_sensor) : 0;
+    const long long nb = 2 + (nword + ns + PHX_SETUP_WORDS - 1) / PHX_SETUP_WORDS;
+    k_call_setup<<<(unsigned)nb, 1024, 0, st>>>(gs, G, gs_off, (unsigned long long)event_index, e->jump_digit.p, jump4, counters, status,
+                                                hitword, nword, sensor, ns);
+}
 
 // every device operation of one plain simulate call on st, then the D2H of num_hit/status
 // into the engine's pinned words; the caller synchronises
@@ -1544,11 +1589,8 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
                          uint32_t* sensor, bool want_hits, cudaStream_t st, bool wave_ok = false)
 {
     const long long nword = (N + 31) / 32;
-    PHX_CU(cudaMemsetAsync(b.status, 0, sizeof(unsigned), st));
-    PHX_CU(cudaMemsetAsync(b.counters, 0, 2 * sizeof(long long), st));
-    k_genstep_offsets<<<1, 1024, 0, st>>>(reinterpret_cast<const float4*>(d_gs), G, b.gs_off);
-    if (event_index > 0) k_jump_build<<<1, 160, 0, st>>>(nullptr, (unsigned long long)event_index, e->jump_pow.p, b.jump);
-    if (event_index > 0 && b.jump4) k_jump_nibbles<<<(PHX_JUMP_BITS / 4 * 16 + 127) / 128, 128, 0, st>>>(b.jump, b.jump4);
+    call_setup(e, reinterpret_cast<const float4*>(d_gs), G, b.gs_off, event_index, b.jump4, b.counters, b.status,
+               want_hits ? b.hitword : nullptr, nword, sensor, st);
     PHX_CU(cudaGetLastError());
     SimArgs a;
     a.S = scene_of(e, e->cfg.root_polish);
@@ -1563,8 +1605,7 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
     a.skip = e->cfg.skipahead_event_offset;
     a.rng = e->rng.p;
     a.rng_slots = e->rng_slots;
-    a.jump = event_index > 0 ? b.jump : nullptr;
-    a.jump4 = event_index > 0 ? b.jump4 : nullptr;
+    a.jump4 = b.jump4;
     a.photon = photon;
     a.seq = seq;
     a.hitword = want_hits ? b.hitword : nullptr;
@@ -1573,7 +1614,6 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
     if (N > 0 && (e->cfg.kernel_mode == 1 || e->cfg.kernel_mode == 2)) {
         // persistent threads with per-lane refill (phx_persist.cuh), or the wavefront rounds
         // (phx_wave.cuh); hit bits are OR-ed in
-        if (want_hits) PHX_CU(cudaMemsetAsync(b.hitword, 0, sizeof(uint32_t) * (size_t)nword, st));
         PersistArgs A = persist_args_from(e, a);
         A.queue = reinterpret_cast<unsigned long long*>(b.counters + 1);
         A.regroup = e->cfg.regroup;
@@ -1592,15 +1632,14 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
         e->last_rounds = 0;
         int rc = wave ? launch_wave(e, A, st) : launch_persistent(e, A, e->cfg.block, st);
         if (rc) return rc;
-        e->last_launches = 1 + (event_index > 0 ? (b.jump4 ? 2 : 1) : 0) + (A.ev_rng ? 1 : 0) +
+        e->last_launches = 1 + (A.ev_rng ? 1 : 0) +
                            (wave ? e->last_wave_launches : 1) + (want_hits ? 3 : 0);
     } else if (N > 0) {
         launch_simulate(e, a, N, st);
         PHX_CU(cudaGetLastError());
         e->last_rounds = 0;
-        e->last_launches = 1 + (event_index > 0 ? (b.jump4 ? 2 : 1) : 0) + 1 + (want_hits ? 3 : 0);
+        e->last_launches = 1 + 1 + (want_hits ? 3 : 0);
     }
-    if (sensor) PHX_CU(cudaMemsetAsync(sensor, 0, sizeof(uint32_t) * std::max(0, e->cfg.num_sensor), st));
     if (want_hits && N > 0) {
         const long long nblock = (nword + 255) / 256;
         k_word_scan<<<(unsigned)nblock, 256, 0, st>>>(b.hitword, nword, b.wordoff, b.blocksum);
@@ -1633,9 +1672,7 @@ static int simulate_device_impl(phx_engine* e, const float* d_gs, int G, long lo
     PHX_CU(e->hitword.ensure((size_t)std::max<long long>(1, nword)));
     PHX_CU(e->wordoff.ensure((size_t)std::max<long long>(1, nword)));
     PHX_CU(e->blocksum.ensure((size_t)std::max<long long>(1, (nword + 255) / 256)));
-    PHX_CU(e->jump_tab.ensure(PHX_JUMP_MATW));
-    PHX_CU(e->jump4.ensure(PHX_JUMP_NIBW));
-    PhxPlainBufs b = { e->gs_off.p, e->hitword.p, e->wordoff.p, e->blocksum.p, e->counters.p, e->status.p, e->jump_tab.p, e->jump4.p };
+    PhxPlainBufs b = { e->gs_off.p, e->hitword.p, e->wordoff.p, e->blocksum.p, e->counters.p, e->status.p, e->jump4.p };
     rc = plain_enqueue(e, b, d_gs, G, N, event_index, photon_offset, photon, d_seq, d_hit, hit_capacity, d_sensor, want_hits, st,
                        true);
     if (rc) return rc;
@@ -1812,8 +1849,7 @@ static int batched_enqueue(phx_engine* e, const PhxBatchCall& c, phx_photon* pho
     k_genstep_offsets<<<1, 1024, 0, st>>>(reinterpret_cast<const float4*>(c.gs), G, e->gs_off.p);
     if (G > 0) {
         k_event_starts<<<(G + 255) / 256, 256, 0, st>>>(c.ev, e->gs_off.p, G, e->ev_start.p);
-        k_jump_build<<<G, 160, 0, st>>>(c.ev, 0ull, e->jump_pow.p, e->jump_tab.p);
-        k_jump_nibbles<<<dim3((PHX_JUMP_BITS / 4 * 16 + 127) / 128, (unsigned)G), 128, 0, st>>>(e->jump_tab.p, e->jump4.p);
+        k_jump_tables<<<G, PHX_JUMP_THREADS, 0, st>>>(c.ev, e->jump_digit.p, e->jump4.p);
     }
     PHX_CU(cudaGetLastError());
     if (want_hits) PHX_CU(cudaMemsetAsync(e->hitword.p, 0, sizeof(uint32_t) * (size_t)std::max<long long>(1, nword), st));
@@ -1836,7 +1872,6 @@ static int batched_enqueue(phx_engine* e, const PhxBatchCall& c, phx_photon* pho
     a.skip = e->cfg.skipahead_event_offset;
     a.rng = e->rng.p;
     a.rng_slots = e->rng_slots;
-    a.jump = e->jump_tab.p;
     a.jump4 = e->jump4.p;
     a.photon = photon;
     a.seq = reinterpret_cast<phx_seq*>(c.seq);
@@ -1914,7 +1949,6 @@ int phx_simulate_batched_device(phx_engine* e, const float* d_gensteps, const in
     }
     if (c.num_event > 0) PHX_CU(e->ev_left.ensure((size_t)c.num_event));
     if (N > 0 && N <= PHX_EV_RNG_MAX) PHX_CU(e->ev_rng.ensure((size_t)N * 6));
-    PHX_CU(e->jump_tab.ensure((size_t)std::max(1, c.G) * PHX_JUMP_MATW));
     PHX_CU(e->jump4.ensure((size_t)std::max(1, c.G) * PHX_JUMP_NIBW));
     // the wavefront loop is capturable when its schedule is fixed (wave_rounds) and the pool holds
     // every photon of the call (no refill rounds, which the host drives)
@@ -1928,7 +1962,7 @@ int phx_simulate_batched_device(phx_engine* e, const float* d_gensteps, const in
             PHX_CU(e->wfree.ensure((size_t)pool));
         }
         const void* bufs[PHX_BATCH_BUFS] = { e->hitword.p, e->wordoff.p, e->blocksum.p, e->gs_off.p, e->ev_start.p, e->ev_left.p,
-                                             e->counters.p, e->status.p, e->photon.p, e->rng.p, e->jump_tab.p, e->ev_rng.p, e->jump4.p,
+                                             e->counters.p, e->status.p, e->photon.p, e->rng.p, e->ev_rng.p, e->jump4.p,
                                              e->wslot.p, e->wprd.p, e->wsidx.p, e->wact0.p, e->wact1.p, e->wcnt.p, e->wfree.p };
         const bool reuse = e->batch_exec && e->batch_call == c && e->batch_launch == launch_key(e) &&
                            memcmp(bufs, e->batch_bufs, sizeof(bufs)) == 0;
@@ -2019,17 +2053,10 @@ int phx_adjoint_device(phx_engine* e, const float* d_gensteps, int32_t num_genst
     const long long N = num_photon;
     PHX_CU(e->gs_off.ensure((size_t)G + 1));
     PHX_CU(e->counters.ensure(8));
-    PHX_CU(e->jump_tab.ensure(PHX_JUMP_MATW));
-    PHX_CU(cudaMemsetAsync(e->status.p, 0, sizeof(unsigned), st));
-    PHX_CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(long long), st));
     PHX_CU(cudaMemsetAsync(d_hits, 0, sizeof(double) * (size_t)e->cfg.num_sensor, st));
     PHX_CU(cudaMemsetAsync(d_grad, 0, sizeof(double) * (size_t)e->cfg.num_sensor * 32, st));
-    k_genstep_offsets<<<1, 1024, 0, st>>>(reinterpret_cast<const float4*>(d_gensteps), G, e->gs_off.p);
-    PHX_CU(e->jump4.ensure(PHX_JUMP_NIBW));
-    if (event_index > 0) {
-        k_jump_build<<<1, 160, 0, st>>>(nullptr, (unsigned long long)event_index, e->jump_pow.p, e->jump_tab.p);
-        k_jump_nibbles<<<(PHX_JUMP_BITS / 4 * 16 + 127) / 128, 128, 0, st>>>(e->jump_tab.p, e->jump4.p);
-    }
+    call_setup(e, reinterpret_cast<const float4*>(d_gensteps), G, e->gs_off.p, event_index, e->jump4.p, e->counters.p, e->status.p,
+               nullptr, 0, nullptr, st);
     PHX_CU(cudaGetLastError());
     SimArgs a;
     a.S = scene_of(e, 0);
@@ -2045,8 +2072,7 @@ int phx_adjoint_device(phx_engine* e, const float* d_gensteps, int32_t num_genst
     a.skip = e->cfg.skipahead_event_offset;
     a.rng = e->rng.p;
     a.rng_slots = e->rng_slots;
-    a.jump = event_index > 0 ? e->jump_tab.p : nullptr;
-    a.jump4 = event_index > 0 ? e->jump4.p : nullptr;
+    a.jump4 = e->jump4.p;
     a.photon = nullptr;
     a.seq = nullptr;
     a.hitword = nullptr;
@@ -2084,8 +2110,7 @@ int phx_adjoint_device(phx_engine* e, const float* d_gensteps, int32_t num_genst
 // Some callers cannot allocate device memory per call: a framework whose caching allocator owns
 // every device byte, or a per-event loop that cannot afford the device-wide synchronisation that
 // cudaMalloc/cudaFree may imply.  phx_simulate_device_noalloc serves them: its scratch (genstep
-// offsets, hit bit words and their prefix sums, counters, status, the event jump matrix and its
-// 4-bit group tables) lives in one fixed file-scope device array instead of engine buffers that
+// offsets, hit bit words and their prefix sums, counters, status, the event's jump tables) lives in one fixed file-scope device array instead of engine buffers that
 // grow on demand.  The array below is sized for PHX_NOALLOC_MAX_PHOTON photons and
 // PHX_NOALLOC_MAX_GENSTEP gensteps per call (about 2.6 MB) and is held on every GPU that loads
 // this library until the process exits.  The bounce loop is always the one-kernel form (the
@@ -2103,7 +2128,6 @@ struct PhxNoAllocScratch {
     uint32_t blocksum[PHX_NOALLOC_BLOCKS];
     long long counters[8];
     unsigned status[8];
-    __align__(16) uint32_t jump[PHX_JUMP_MATW];
     __align__(16) uint32_t jump4[PHX_JUMP_NIBW];
 };
 
@@ -2159,8 +2183,7 @@ extern "C" int phx_simulate_device_noalloc(phx_engine* e, const float* d_genstep
     const long long N = num_photon;
     // phx_simulate_device's launch sequence in its one-kernel loop form (never the wavefront
     // rounds), on the fixed scratch
-    PhxPlainBufs b = { scr->gs_off, scr->hitword, scr->wordoff, scr->blocksum, scr->counters, scr->status, scr->jump,
-                       scr->jump4 };
+    PhxPlainBufs b = { scr->gs_off, scr->hitword, scr->wordoff, scr->blocksum, scr->counters, scr->status, scr->jump4 };
     rc = plain_enqueue(e, b, d_gensteps, num_genstep, N, event_index, photon_offset, reinterpret_cast<phx_photon*>(d_out->photon),
                        reinterpret_cast<phx_seq*>(d_out->seq), reinterpret_cast<phx_photon*>(d_out->hit), d_out->hit_capacity,
                        d_out->sensor_hits, want_hits, st);

@@ -369,30 +369,9 @@ PHX_D int phx_find_genstep(const long long* off, int G, long long idx)
     return lo;
 }
 
-// Advance a loaded XORWOW state by n steps with a precomputed jump matrix M (= T^n, see
-// phx_rngjump.h): v <- M v over GF(2), d <- d + 362437 n.  Same state as skipahead(n).
-PHX_D void phx_rng_jump(curandStateXORWOW& s, const uint32_t* __restrict__ M, unsigned long long n)
-{
-    uint32_t o0 = 0u, o1 = 0u, o2 = 0u, o3 = 0u, o4 = 0u;
-    const uint32_t in[5] = { s.v[0], s.v[1], s.v[2], s.v[3], s.v[4] };
-#pragma unroll 1
-    for (int w = 0; w < 5; w++) {
-        const uint32_t x = in[w];
-        const uint32_t* colw = M + (size_t)(32 * w) * 8;
-#pragma unroll 8
-        for (int b = 0; b < 32; b++) {
-            const uint32_t m = 0u - ((x >> b) & 1u);
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(colw + 8 * b));
-            const uint32_t e4 = __ldg(colw + 8 * b + 4);
-            o0 ^= a.x & m; o1 ^= a.y & m; o2 ^= a.z & m; o3 ^= a.w & m; o4 ^= e4 & m;
-        }
-    }
-    s.v[0] = o0; s.v[1] = o1; s.v[2] = o2; s.v[3] = o3; s.v[4] = o4;
-    s.d += (unsigned int)((362437ull * n) & 0xffffffffull);
-}
-
-// v <- M v through the 4-bit group tables of M (k_jump_nibbles): 40 lookups instead of 160 column
-// steps, the same XOR of the same columns, so the same state as phx_rng_jump and skipahead(n)
+// Advance a loaded XORWOW state by n steps: v <- M v over GF(2) with M = T^n (phx_rngjump.h), d <- d +
+// 362437 n.  M comes as 4-bit group tables (phx_event_table): 40 lookups, each the XOR of up to four
+// columns.  Same state as skipahead(n).
 PHX_D void phx_rng_jump4(curandStateXORWOW& s, const uint32_t* __restrict__ T, unsigned long long n)
 {
     uint32_t o0 = 0u, o1 = 0u, o2 = 0u, o3 = 0u, o4 = 0u;
@@ -412,48 +391,104 @@ PHX_D void phx_rng_jump4(curandStateXORWOW& s, const uint32_t* __restrict__ T, u
     s.d += (unsigned int)((362437ull * n) & 0xffffffffull);
 }
 
-// the 4-bit group tables of jump matrix blockIdx.y of M (one per genstep in batched calls):
-// thread t builds entry (t / 16, t % 16)
-__global__ void k_jump_nibbles(const uint32_t* __restrict__ M, uint32_t* T)
+// The event's jump matrix as 4-bit group tables, by one block of at least PHX_JUMP_THREADS threads.
+// The event index is taken as hex digits: D holds, for digit position g and value v in 1..15, the
+// group tables of T^(skip v 16^g) (k_jump_digits), and M is their product.  Four threads work on a
+// column: the first digit's column is a table entry, each further digit is 40 lookups, ten a thread.
+// `col`: 160 x 5 words of shared memory.  Bound by the latency of one dependent round of L2 lookups a
+// digit: event indices up to 4095 take 5 us where composing the matrix column by column took 48.
+#define PHX_JUMP_THREADS 640
+PHX_D void phx_event_table(unsigned long long event, const uint32_t* __restrict__ D, uint32_t* T, uint32_t* col)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= PHX_JUMP_BITS / 4 * 16) return;
-    M += (size_t)blockIdx.y * PHX_JUMP_MATW;
-    T += (size_t)blockIdx.y * PHX_JUMP_NIBW;
-    const int g = t >> 4, k = t & 15;
-    uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
-    for (int b = 0; b < 4; b++) {
-        if (!((k >> b) & 1)) continue;
-        const uint32_t* col = M + (size_t)(4 * g + b) * PHX_JUMP_COLW;
-        for (int q = 0; q < 5; q++) o[q] ^= col[q];
+    const int t = threadIdx.x;
+    if (t < PHX_JUMP_THREADS) {
+        const int c = t >> 2, part = t & 3;
+        uint32_t v[5] = { 0u, 0u, 0u, 0u, 0u };
+        v[c >> 5] = 1u << (c & 31);
+        bool first = true;
+        for (int g = 0; g < PHX_JUMP_DIGITS; g++) {
+            const unsigned x = (unsigned)(event >> (4 * g)) & 15u;
+            if (!x) continue;
+            const uint32_t* E = D + (size_t)(15 * g + (int)x - 1) * PHX_JUMP_NIBW;
+            if (first) {
+                const uint32_t* e = E + (size_t)((c >> 2) * 16 + (1 << (c & 3))) * PHX_JUMP_COLW;
+                const uint4 a = __ldg(reinterpret_cast<const uint4*>(e));
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = __ldg(e + 4);
+                first = false;
+                continue;
+            }
+            uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
+#pragma unroll
+            for (int w = 0; w < 5; w++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {            // groups 2 part and 2 part + 1 of word w
+                    const int q = 2 * part + h;
+                    const uint32_t* e = E + (size_t)((8 * w + q) * 16 + (int)((v[w] >> (4 * q)) & 15u)) * PHX_JUMP_COLW;
+                    const uint4 a = __ldg(reinterpret_cast<const uint4*>(e));
+                    const uint32_t e4 = __ldg(e + 4);
+                    o[0] ^= a.x; o[1] ^= a.y; o[2] ^= a.z; o[3] ^= a.w; o[4] ^= e4;
+                }
+#pragma unroll
+            for (int w = 0; w < 5; w++) {
+                o[w] ^= __shfl_xor_sync(0xffffffffu, o[w], 1);
+                v[w] = o[w] ^ __shfl_xor_sync(0xffffffffu, o[w], 2);
+            }
+        }
+        if (part == 0)
+            for (int w = 0; w < 5; w++) col[5 * c + w] = v[w];
     }
-    uint32_t* dst = T + (size_t)t * PHX_JUMP_COLW;
-    for (int q = 0; q < 5; q++) dst[q] = o[q];
-    dst[5] = dst[6] = dst[7] = 0u;
+    __syncthreads();
+    if (t < PHX_JUMP_BITS / 4 * 16) {
+        const int g = t >> 4, k = t & 15;
+        uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
+        for (int b = 0; b < 4; b++) {
+            const uint32_t m = 0u - ((unsigned)(k >> b) & 1u);
+            for (int w = 0; w < 5; w++) o[w] ^= col[5 * (4 * g + b) + w] & m;
+        }
+        uint4* dst = reinterpret_cast<uint4*>(T + (size_t)t * PHX_JUMP_COLW);
+        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[1] = make_uint4(o[4], 0u, 0u, 0u);
+    }
 }
 
-// one event jump matrix per entry: entry i uses event ev[i] (or `single` when ev is null);
-// thread c composes column c of prod_k P_k^(bit k of event)
-__global__ void k_jump_build(const int* ev, unsigned long long single, const uint32_t* __restrict__ P, uint32_t* out)
+// the digit tables of phx_event_table from the powers P_k = T^(skip 2^k): block 15 g + v - 1 composes
+// the columns of T^(skip v 16^g) (once per engine)
+__global__ void __launch_bounds__(PHX_JUMP_THREADS) k_jump_digits(const uint32_t* __restrict__ P, uint32_t* D)
 {
-    const int c = threadIdx.x;
-    if (c >= 160) return;
-    const unsigned long long e = ev ? (unsigned long long)(unsigned)ev[blockIdx.x] : single;
-    uint32_t v[5] = { 0u, 0u, 0u, 0u, 0u };
-    v[c >> 5] = 1u << (c & 31);
-    for (int k = 0; k < 32; k++) {
-        if (!((e >> k) & 1ull)) continue;
-        const uint32_t* Pk = P + (size_t)k * 160 * 8;
-        uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
-        for (int bit = 0; bit < 160; bit++) {
-            if ((v[bit >> 5] >> (bit & 31)) & 1u)
-                for (int q = 0; q < 5; q++) o[q] ^= Pk[bit * 8 + q];
+    __shared__ uint32_t col[PHX_JUMP_BITS * 5];
+    const int g = blockIdx.x / 15, x = blockIdx.x % 15 + 1, t = threadIdx.x;
+    if (t < PHX_JUMP_BITS) {
+        uint32_t v[5] = { 0u, 0u, 0u, 0u, 0u };
+        v[t >> 5] = 1u << (t & 31);
+        for (int k = 0; k < 4; k++) {
+            if (!((x >> k) & 1)) continue;
+            const uint32_t* Pk = P + (size_t)(4 * g + k) * PHX_JUMP_MATW;
+            uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
+            for (int bit = 0; bit < PHX_JUMP_BITS; bit++) {
+                const uint32_t m = 0u - ((v[bit >> 5] >> (bit & 31)) & 1u);
+                for (int q = 0; q < 5; q++) o[q] ^= Pk[bit * PHX_JUMP_COLW + q] & m;
+            }
+            for (int q = 0; q < 5; q++) v[q] = o[q];
         }
-        for (int q = 0; q < 5; q++) v[q] = o[q];
+        for (int q = 0; q < 5; q++) col[5 * t + q] = v[q];
     }
-    uint32_t* dst = out + (size_t)blockIdx.x * 160 * 8 + c * 8;
-    for (int q = 0; q < 5; q++) dst[q] = v[q];
-    dst[5] = dst[6] = dst[7] = 0u;
+    __syncthreads();
+    if (t < PHX_JUMP_BITS / 4 * 16) {
+        uint32_t o[5] = { 0u, 0u, 0u, 0u, 0u };
+        for (int b = 0; b < 4; b++) {
+            const uint32_t m = 0u - ((unsigned)((t & 15) >> b) & 1u);
+            for (int w = 0; w < 5; w++) o[w] ^= col[5 * (4 * (t >> 4) + b) + w] & m;
+        }
+        uint32_t* dst = D + (size_t)blockIdx.x * PHX_JUMP_NIBW + (size_t)t * PHX_JUMP_COLW;
+        for (int q = 0; q < 8; q++) dst[q] = q < 5 ? o[q] : 0u;
+    }
+}
+
+// the tables of every genstep's event (batched calls): one block per genstep
+__global__ void __launch_bounds__(PHX_JUMP_THREADS) k_jump_tables(const int* ev, const uint32_t* __restrict__ D, uint32_t* T)
+{
+    __shared__ uint32_t col[PHX_JUMP_BITS * 5];
+    phx_event_table((unsigned long long)(unsigned)ev[blockIdx.x], D, T + (size_t)blockIdx.x * PHX_JUMP_NIBW, col);
 }
 
 PHX_D void phx_load_rng(curandStateXORWOW& s, const uint32_t* rng, long long slots, long long slot)

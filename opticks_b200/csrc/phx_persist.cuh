@@ -30,8 +30,7 @@ struct PersistArgs {
     unsigned long long seed, rng_offset;   // curand_init arguments for photons beyond the prepared slots
     const uint32_t* rng;
     long long rng_slots;
-    const uint32_t* jump;           // event jump matrices: one (single event) or one per genstep (batched)
-    const uint32_t* jump4;          // the 4-bit group tables of those matrices (same indexing), or null
+    const uint32_t* jump4;          // event jump tables (phx_event_table): one (single event) or one per genstep (batched)
     const uint32_t* ev_rng;         // optional: XORWOW states already advanced to each photon's event
     long long ev_rng_n;             //   (six planes of ev_rng_n words, by photon index; k_rng_event)
     phx_photon* photon;
@@ -216,9 +215,7 @@ PHX_D void phx_event_rng(curandStateXORWOW& s, const PersistArgs& A, int gi, lon
     }
     if (ev > 0ull) {
         if (planes) phx_rng_jump4_planes(s, planes, A.skip * ev);
-        else if (A.jump4) phx_rng_jump4(s, A.jump4 + (A.gs_event ? (size_t)gi * PHX_JUMP_NIBW : 0), A.skip * ev);
-        else if (A.jump) phx_rng_jump(s, A.jump + (A.gs_event ? (size_t)gi * PHX_JUMP_MATW : 0), A.skip * ev);
-        else skipahead(A.skip * ev, &s);
+        else phx_rng_jump4(s, A.jump4 + (A.gs_event ? (size_t)gi * PHX_JUMP_NIBW : 0), A.skip * ev);
     }
 }
 

@@ -6,18 +6,19 @@
 //     t = x ^ (x >> 2); x = y; y = z; z = w; w = v; v = (v ^ (v << 4)) ^ (t ^ (t << 1)); d += 362437
 // The five-word part is linear over GF(2), so n steps are one 160x160 bit matrix T^n, and the
 // counter advances by 362437 n.  The host builds T from the recurrence, the powers
-// P_k = T^(skip * 2^k) by repeated squaring, and the device composes M_e = prod_k P_k^(bit k of e)
-// once per event (one thread per matrix column).  A photon then applies M_e to its 160-bit state:
-// 160 predicated XORs of 32-byte columns instead of a multi-stage skipahead per photon, or, for a
-// single event, 40 lookups in tables of M_e over 4-bit groups of the state (the "four Russians"
-// grouping of a GF(2) matrix-vector product), built once per call.
+// P_k = T^(skip * 2^k) by repeated squaring.  At engine creation the device turns them into tables of
+// T^(skip * v * 16^g) for every hex digit g and value v (k_jump_digits), and a call composes its
+// event's matrix M_e from the tables of the event's non-zero digits (phx_event_table), as tables of
+// M_e over 4-bit groups of the state (the "four Russians" grouping of a GF(2) matrix-vector
+// product).  A photon then advances its 160-bit state by 40 lookups, instead of a multi-stage
+// skipahead per photon.
 // Matrices are stored column-major, one column = the image of one state bit, padded to 8 words.
 #pragma once
 #include <stdint.h>
 #include <vector>
 
 #include "phx_pod.h"                        // PHX_JUMP_BITS, PHX_JUMP_COLW, PHX_JUMP_MATW
-#define PHX_JUMP_POWERS 32                       // events < 2^32
+#define PHX_JUMP_POWERS (4 * PHX_JUMP_DIGITS)
 
 struct PhxV5 { uint32_t w[5]; };
 

@@ -307,7 +307,7 @@ PHX_D bool wave_refill(PhxLane& L, const PersistArgs& A, bool need, unsigned& st
 PHX_D const uint32_t* wave_jump_planes(const PersistArgs& A)
 {
     __shared__ uint32_t planes[5 * PHX_JUMP_PLANE];
-    if (!A.jump4 || A.gs_event || A.ev_rng || A.event_index == 0ull) return nullptr;
+    if (A.gs_event || A.ev_rng || A.event_index == 0ull) return nullptr;
     phx_jump_planes_load(planes, A.jump4);
     __syncthreads();
     return planes;
