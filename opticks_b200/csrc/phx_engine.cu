@@ -432,6 +432,45 @@ __global__ void k_compact(const phx_photon* photon, long long N, const uint32_t*
     }
 }
 
+// The same for at most PHX_COMPACT_WORDS hit words in one launch: each block counts the bits before its
+// own 32 words itself (8 words a thread in the last block at most), so no scan kernels run ahead of
+// it: one launch of 5 us for three of 14 us.  Beyond that the counting grows with the square of the words.
+#define PHX_COMPACT_WORDS 8192
+__global__ void __launch_bounds__(1024) k_compact_small(const phx_photon* photon, long long N, const uint32_t* word, int nword,
+                                                        phx_photon* hit, long long hit_capacity, uint32_t* sensor, int num_sensor,
+                                                        long long* total, unsigned* status)
+{
+    __shared__ uint32_t part[32], mine[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int w0 = blockIdx.x * 32, w = w0 + wid;
+    const uint32_t bits = w < nword ? word[w] : 0u;
+    uint32_t c = 0u;
+    for (int k = threadIdx.x; k < w0; k += 1024) c += __popc(word[k]);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) { part[wid] = c; mine[wid] = __popc(bits); }
+    __syncthreads();
+    uint32_t before = __reduce_add_sync(0xffffffffu, part[lane] + (lane < wid ? mine[lane] : 0u));
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 1023) *total = (long long)before + __popc(bits);
+    if (!((bits >> lane) & 1u)) return;
+    const long long idx = 32ll * w + lane;
+    if (idx >= N) return;
+    const long long dst = (long long)before + __popc(bits & ((1u << lane) - 1u));
+    const float4* src = reinterpret_cast<const float4*>(photon + idx);
+    const float4 q0 = src[0], q1 = src[1], q2 = src[2], q3 = src[3];
+    if (hit) {
+        if (dst < hit_capacity) {
+            float4* o = reinterpret_cast<float4*>(hit + dst);
+            o[0] = q0; o[1] = q1; o[2] = q2; o[3] = q3;
+        } else {
+            atomicOr(status, (unsigned)PHX_STATUS_HIT_OVERFLOW);
+        }
+    }
+    if (sensor) {
+        const unsigned id = __float_as_uint(q3.y) & 0xffffffu;
+        if (id > 0u && (int)(id - 1u) < num_sensor) atomicAdd(sensor + (id - 1u), 1u);
+    }
+}
+
 // CSGScan : one thread per ray, SoA rays
 template <int CV>
 __global__ void k_csg_scan(PhxCsgCtx csg, int root, float t_min, const float* rays, long long n, float4* out, unsigned* status)
@@ -1365,6 +1404,13 @@ static long long wave_pool_for(const phx_engine* e, long long N, bool adj)
     }
     return std::max<long long>(1, std::min(std::min(N, pool), PHX_WAVE_POOL_MAX));
 }
+// Calls of at most this many photons skip the rounds: all their paths fit in the tail kernel's resident
+// lanes (56,832 of them), so a round's two launches only add to the latency of the longest path.
+// Detector events: 1,000 photons 140 us with two rounds, 118 without; 50k 242 / 217; 200k 469 / 475 (there
+// the coherent rounds pay again).
+#ifndef PHX_WAVE_SMALL
+#define PHX_WAVE_SMALL 65536
+#endif
 // calls of at most this many photons get their event-advanced RNG states in one coherent pass
 // ahead of the loop (24 B per photon of scratch); larger ones advance each state as it starts
 #define PHX_EV_RNG_MAX (1LL << 26)
@@ -1431,8 +1477,9 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
     W.live_bits = refill ? e->wlive.p : nullptr;
     PHX_CU(cudaGetLastError());
     int cur = 0;
-    const int rounds = ADJ ? e->cfg.adj_wave_rounds : e->cfg.wave_rounds;
-    if (rounds > 0 && !refill) {
+    const int cfg_rounds = ADJ ? e->cfg.adj_wave_rounds : e->cfg.wave_rounds;
+    if (cfg_rounds > 0 && !refill) {
+        const int rounds = !ADJ && N <= PHX_WAVE_SMALL ? 0 : cfg_rounds;
         // fixed schedule, no host read: wave_rounds rounds, then the tail kernel finishes whatever is
         // still live (it reads the count on the device; a grid-stride loop over any count), so the
         // whole call can be captured as a CUDA graph
@@ -1589,6 +1636,7 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
                          uint32_t* sensor, bool want_hits, cudaStream_t st, bool wave_ok = false)
 {
     const long long nword = (N + 31) / 32;
+    const int hit_launches = !want_hits ? 0 : nword <= PHX_COMPACT_WORDS ? 1 : 3;
     call_setup(e, reinterpret_cast<const float4*>(d_gs), G, b.gs_off, event_index, b.jump4, b.counters, b.status,
                want_hits ? b.hitword : nullptr, nword, sensor, st);
     PHX_CU(cudaGetLastError());
@@ -1633,14 +1681,18 @@ static int plain_enqueue(phx_engine* e, const PhxPlainBufs& b, const float* d_gs
         int rc = wave ? launch_wave(e, A, st) : launch_persistent(e, A, e->cfg.block, st);
         if (rc) return rc;
         e->last_launches = 1 + (A.ev_rng ? 1 : 0) +
-                           (wave ? e->last_wave_launches : 1) + (want_hits ? 3 : 0);
+                           (wave ? e->last_wave_launches : 1) + hit_launches;
     } else if (N > 0) {
         launch_simulate(e, a, N, st);
         PHX_CU(cudaGetLastError());
         e->last_rounds = 0;
-        e->last_launches = 1 + 1 + (want_hits ? 3 : 0);
+        e->last_launches = 1 + 1 + hit_launches;
     }
-    if (want_hits && N > 0) {
+    if (want_hits && N > 0 && nword <= PHX_COMPACT_WORDS) {
+        k_compact_small<<<(unsigned)((nword + 31) / 32), 1024, 0, st>>>(photon, N, b.hitword, (int)nword, hit, hcap, sensor,
+                                                                        e->cfg.num_sensor, b.counters, b.status);
+        PHX_CU(cudaGetLastError());
+    } else if (want_hits && N > 0) {
         const long long nblock = (nword + 255) / 256;
         k_word_scan<<<(unsigned)nblock, 256, 0, st>>>(b.hitword, nword, b.wordoff, b.blocksum);
         k_block_scan<<<1, 1024, 0, st>>>(b.blocksum, (int)nblock, b.counters);
