@@ -444,6 +444,21 @@ PHX_COLD float4 leaf_torus(const float4 q0, const float t_min, const float3 o, c
     const double s_min = (double)t_min * dl;
     if (s_out <= s_min) return isect;
     const double s0 = fmax(s_in, 0.0);
+    {
+        // The torus lies in the slab |z| <= r outside the cylinder R - r.  The stretch of the ray that
+        // the bounding sphere and the slab leave has no root when it is empty or when both its ends,
+        // and so all of it, lie in the hole (margins far beyond FP64 error).
+        const double rp = r * (1.0 + 1e-9) + 1e-9 * Rb, hole = (R - rp) * (1.0 - 1e-9);
+        double a = fmax(s0, s_min) - 1e-9 * Rb, b = s_out + 1e-9 * Rb;
+        if (nz != 0.0) {
+            const double iz = 1.0 / nz, za = (-rp - oz) * iz, zb = (rp - oz) * iz;
+            a = fmax(a, fmin(za, zb));
+            b = fmin(b, fmax(za, zb));
+        } else if (fabs(oz) > rp) return isect;
+        if (a > b) return isect;
+        const double xa = ox + a * nx, ya = oy + a * ny, xb = ox + b * nx, yb = oy + b * ny;
+        if (hole > 0.0 && xa * xa + ya * ya < hole * hole && xb * xb + yb * yb < hole * hole) return isect;
+    }
     ox += s0 * nx; oy += s0 * ny; oz += s0 * nz;
     const double B = 2.0 * (ox * nx + oy * ny + oz * nz);
     const double C = ox * ox + oy * oy + oz * oz + R * R - r * r;

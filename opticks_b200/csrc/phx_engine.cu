@@ -106,6 +106,7 @@ struct phx_engine {
     int last_tail = 0;        // the last wavefront call finished its paths in one tail kernel
     long long last_wave_launches = 0;   // kernel launches of the last wavefront loop
     std::vector<int> prim_node_offset;
+    std::vector<float4> prim_ball;         // per prim: a ball around all it can hit (phx_ball_missed)
     // physics
     cudaArray_t bnd_arr = nullptr, icdf_arr = nullptr, planck_arr = nullptr;
     cudaTextureObject_t bnd_tex = 0, icdf_tex = 0, planck_tex = 0;
@@ -471,18 +472,58 @@ __global__ void __launch_bounds__(1024) k_compact_small(const phx_photon* photon
     }
 }
 
-// CSGScan : one thread per ray, SoA rays
+// CSGScan (SoA rays).  Most rays of a scan pass the prim by, and a boolean tree costs thousands of
+// instructions: a warp first tests windows of 32 rays against the prim's bounding ball (phx_ball_missed,
+// never true of a ray the tree would hit) and queues the others, then evaluates the tree for 32 queued
+// rays at a time, so no lane idles beside an early miss.
 template <int CV>
-__global__ void k_csg_scan(PhxCsgCtx csg, int root, float t_min, const float* rays, long long n, float4* out, unsigned* status)
+__global__ void __launch_bounds__(128) k_csg_scan(PhxCsgCtx csg, int root, float t_min, float4 ball, const float* rays, long long n,
+                                                  float4* out, unsigned* status)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float3 o = make_float3(__ldg(rays + i), __ldg(rays + n + i), __ldg(rays + 2 * n + i));
-    const float3 d = make_float3(__ldg(rays + 3 * n + i), __ldg(rays + 4 * n + i), __ldg(rays + 5 * n + i));
-    unsigned st = 0;
-    float4 is;
-    const bool valid = intersect_prim<CV>(is, csg, root, t_min, o, d, st);
-    out[i] = valid ? is : make_float4(0.f, 0.f, 0.f, 0.f);
+    __shared__ float qray[4][6][64];
+    __shared__ long long qidx[4][64];
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const long long warps = 4ll * gridDim.x;
+    const long long width = min(32ll, (n + warps - 1) / warps);      // few rays: spread over all warps
+    long long at = width * ((long long)blockIdx.x * 4 + w);
+    const long long stride = width * warps;
+    unsigned waiting = 0u, st = 0u;
+    for (;;) {
+        while (waiting < 32u && at < n) {
+            const long long i = at + lane;
+            at += stride;
+            bool keep = false;
+            float r[6];
+            if ((long long)lane < width && i < n) {
+#pragma unroll
+                for (int k = 0; k < 6; k++) r[k] = __ldg(rays + k * n + i);
+                keep = !phx_ball_missed(ball, make_float3(r[0], r[1], r[2]), make_float3(r[3], r[4], r[5]), t_min);
+                if (!keep) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            const unsigned m = __ballot_sync(FULL, keep);
+            if (keep) {
+                const unsigned q = waiting + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+                for (int k = 0; k < 6; k++) qray[w][k][q] = r[k];
+                qidx[w][q] = i;
+            }
+            waiting += __popc(m);
+            __syncwarp();
+        }
+        if (waiting == 0u) break;
+        const unsigned take = min(waiting, 32u);
+        waiting -= take;
+        if (lane < take) {
+            const unsigned q = waiting + lane;
+            const float3 o = make_float3(qray[w][0][q], qray[w][1][q], qray[w][2][q]);
+            const float3 d = make_float3(qray[w][3][q], qray[w][4][q], qray[w][5][q]);
+            float4 is;
+            const bool valid = intersect_prim<CV>(is, csg, root, t_min, o, d, st);
+            out[qidx[w][q]] = valid ? is : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+    }
     if (st) atomicOr(status, st);
 }
 
@@ -715,6 +756,29 @@ static const char* check_prim_nodes(const phx_geometry* geo, int root)
         if (m) return m;
     }
     return nullptr;
+}
+
+// A ball around every hit of a prim's own nodes (the caller's prim box plays no part), padded beyond FP32
+// error, for prims made of the five base leaves and the operators; radius 3e38 (nothing is outside)
+// for any other prim and for an unbounded one.
+static float4 scan_ball(const phx_geometry* geo, int p)
+{
+    int32_t nn, no;
+    memcpy(&nn, geo->prim + 16 * (size_t)p + 0, 4);
+    memcpy(&no, geo->prim + 16 * (size_t)p + 1, 4);
+    uint32_t root_tc, num = 1;
+    memcpy(&root_tc, geo->node + 16 * (size_t)no + 14, 4);
+    if (root_tc >= PHX_CSG_UNION && root_tc <= PHX_CSG_DIFFERENCE) memcpy(&num, geo->node + 16 * (size_t)no, 4);   // checked subNum
+    bool base = true;
+    for (uint32_t i = 0; i < num; i++) {
+        uint32_t tc;
+        memcpy(&tc, geo->node + 16 * (size_t)(no + (int)i) + 14, 4);
+        base = base && phx_csg_base_typecode(tc);
+    }
+    const PhxSph s = base ? node_sphere(geo, no, 0, (int)num) : PhxSph{ { 0, 0, 0 }, PHX_SPH_INF };
+    if (!(s.r < 1e30)) return make_float4(0.f, 0.f, 0.f, 3e38f);
+    const double cn = std::sqrt(s.c[0] * s.c[0] + s.c[1] * s.c[1] + s.c[2] * s.c[2]);
+    return make_float4((float)s.c[0], (float)s.c[1], (float)s.c[2], (float)(s.r * (1.0 + 1e-4) + 1e-5 * (cn + s.r) + 1e-3));
 }
 
 // the kind of a prim (PHX_KIND_*): what the closest-hit kernels can evaluate inline
@@ -1150,6 +1214,7 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     std::vector<PhxLeafInput> leaves;
     std::vector<PhxSph> psph((size_t)std::max(1, geo->num_prim));
     for (int p = 0; p < geo->num_prim; p++) psph[p] = prim_sphere(geo, p);
+    for (int p = 0; p < geo->num_prim; p++) e->prim_ball.push_back(scan_ball(geo, p));
     for (int i = 0; i < geo->num_inst; i++) {
         const float* q = geo->inst + 16 * i;
         float m[16];
@@ -1584,11 +1649,16 @@ static int launch_simulate(phx_engine* e, const SimArgs& a, long long N, cudaStr
 }
 
 template <int CV>
-static void launch_scan_t(const PhxCsgCtx& csg, int root, float t_min, const float* d_rays, long long n, float4* out, unsigned* status,
-                          cudaStream_t st)
+static int launch_scan_t(int device, const PhxCsgCtx& csg, int root, float t_min, const float4& ball, const float* d_rays, long long n,
+                         float4* out, unsigned* status, cudaStream_t st)
 {
-    const int B = 128;
-    k_csg_scan<CV><<<(unsigned)((n + B - 1) / B), B, 0, st>>>(csg, root, t_min, d_rays, n, out, status);
+    static int grid[128] = {};
+    if (device < 0 || device >= 128) return phx_fail(-1, "device ordinal %d out of range", device);
+    int rc = wave_grid(k_csg_scan<CV>, device, grid);
+    if (rc) return rc;
+    k_csg_scan<CV><<<(unsigned)std::min<long long>(grid[device], (n + 3) / 4), 128, 0, st>>>(csg, root, t_min, ball, d_rays, n, out,
+                                                                                               status);
+    return 0;
 }
 
 template <int CV>
@@ -1795,12 +1865,12 @@ int phx_csg_scan_device(phx_engine* e, int32_t prim, float t_min, const float* d
     if (n > 0) {
         float4* out = reinterpret_cast<float4*>(d_isect);
         const int root = e->prim_node_offset[prim];
-        switch (cv_of(e, polish != 0)) {
-            case 1: launch_scan_t<1>(csg, root, t_min, d_rays, n, out, e->status.p, st); break;
-            case 2: launch_scan_t<2>(csg, root, t_min, d_rays, n, out, e->status.p, st); break;
-            case 3: launch_scan_t<3>(csg, root, t_min, d_rays, n, out, e->status.p, st); break;
-            default: launch_scan_t<0>(csg, root, t_min, d_rays, n, out, e->status.p, st); break;
-        }
+        const float4 ball = e->prim_ball[prim];
+        const auto launch = [&]() -> int {
+            PHX_CV_RETURN(cv_of(e, polish != 0), (launch_scan_t<CVK>(e->device, csg, root, t_min, ball, d_rays, n, out, e->status.p, st)));
+        };
+        const int rc = launch();
+        if (rc) return rc;
         PHX_CU(cudaGetLastError());
     }
     return 0;
