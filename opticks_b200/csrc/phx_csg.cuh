@@ -1025,6 +1025,7 @@ PHX_D float4 intersect_tree3_fast(const float4* __restrict__ node, const float4*
     float4 L = make_float4(0.f, 0.f, 0.f, 0.f), R = L;
     int which = 1;                  // node evaluated in this turn: root + which
     float t0 = t_min;
+#pragma unroll 1
     for (int it = 0; it < PHX_TREE3_LOOP_CAP + 1; it++) {
         const float4 v = leaf_fast<POLISH>(node, itra, root + which, t0, o, d);
         if (which == 1) L = v; else R = v;

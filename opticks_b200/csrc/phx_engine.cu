@@ -527,22 +527,45 @@ __global__ void __launch_bounds__(128) k_csg_scan(PhxCsgCtx csg, int root, float
     if (st) atomicOr(status, st);
 }
 
+// idle lanes a warp of k_trace_rays waits for before it takes new rays
+#ifndef PHX_TRACE_REFILL
+#define PHX_TRACE_REFILL 12
+#endif
 // The trace step of simtrace (CSGOptiX/CSGOptiX7.cu:563-603 calls trace(), :112-218): the closest
 // hit of arbitrary rays over the whole geometry, one thread per ray (SoA rays), written as the
 // reference's quad2 PRD (sysrap/squad.h:180-245): q0 normal.xyz (world, unnormalised), t;
 // q1 lposcost, 0, iindex<<16|identity, globalPrimIdx<<16|boundary (0xffffffff words: a miss)
 template <int CV>
-__global__ void k_trace_rays(PhxScene S, const float* rays, long long n, float t_min, float t_max, float4* prd_out, unsigned* status)
+__global__ void __launch_bounds__(128, 3) k_trace_rays(PhxScene S, const float* rays, long long n, float t_min, float t_max,
+                                                       float4* prd_out, unsigned* status)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float3 o = make_float3(__ldg(rays + i), __ldg(rays + n + i), __ldg(rays + 2 * n + i));
-    const float3 d = make_float3(__ldg(rays + 3 * n + i), __ldg(rays + 4 * n + i), __ldg(rays + 5 * n + i));
+    __shared__ int2 queue[4 * 64];
+    // windows of 32 rays; with fewer rays than lanes, narrower ones over all warps (less divergence)
+    const long long warps = 4ll * gridDim.x;
+    const long long width = min(32ll, (n + warps - 1) / warps);
+    long long at = width * ((long long)blockIdx.x * 4 + (threadIdx.x >> 5));      // the warp's next window
+    const long long stride = width * warps;
     unsigned st = 0;
-    PhxPRD prd;
-    phx_trace<CV>(S, o, d, t_min, t_max, prd, st);
-    prd_out[2 * i] = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
-    prd_out[2 * i + 1] = make_float4(prd.lposcost, 0.f, __uint_as_float(prd.ii_id), __uint_as_float(prd.gp_bd));
+    phx_trace_stream<CV>(
+        S, t_max, PHX_TRACE_REFILL, queue + 64 * (threadIdx.x >> 5), st,
+        [&]() -> long long {
+            const long long b = at;
+            at += stride;
+            return b < n ? b : -1ll;
+        },
+        [&](long long base, unsigned lane, unsigned& i) {
+            i = (unsigned)(base + lane);
+            return (long long)lane < width && base + lane < n;
+        },
+        [&](unsigned i, float3& o, float3& d, float& tmin) {
+            o = make_float3(__ldg(rays + i), __ldg(rays + n + i), __ldg(rays + 2 * n + i));
+            d = make_float3(__ldg(rays + 3 * n + i), __ldg(rays + 4 * n + i), __ldg(rays + 5 * n + i));
+            tmin = t_min;
+        },
+        [&](unsigned i, const PhxPRD& prd) {
+            prd_out[2 * (size_t)i] = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
+            prd_out[2 * (size_t)i + 1] = make_float4(prd.lposcost, 0.f, __uint_as_float(prd.ii_id), __uint_as_float(prd.gp_bd));
+        });
     if (st) atomicOr(status, st);
 }
 
@@ -1662,17 +1685,21 @@ static int launch_scan_t(int device, const PhxCsgCtx& csg, int root, float t_min
 }
 
 template <int CV>
-static void launch_trace_t(const PhxScene& S, const float* d_rays, long long n, float t_min, float t_max, float4* out, unsigned* status,
+static int launch_trace_t(int device, const PhxScene& S, const float* d_rays, long long n, float t_min, float t_max, float4* out, unsigned* status,
                            cudaStream_t st)
 {
-    const int B = 128;
-    k_trace_rays<CV><<<(unsigned)((n + B - 1) / B), B, 0, st>>>(S, d_rays, n, t_min, t_max, out, status);
+    static int grid[128] = {};
+    if (device < 0 || device >= 128) return phx_fail(-1, "device ordinal %d out of range", device);
+    int rc = wave_grid(k_trace_rays<CV>, device, grid);
+    if (rc) return rc;
+    k_trace_rays<CV><<<(unsigned)std::min<long long>(grid[device], (n + 3) / 4), 128, 0, st>>>(S, d_rays, n, t_min, t_max, out, status);
+    return 0;
 }
 
 static int launch_trace(phx_engine* e, const float* d_rays, long long n, float t_min, float t_max, float4* out, cudaStream_t st)
 {
     const PhxScene S = scene_of(e, e->cfg.root_polish);
-    PHX_CV_RETURN(cv_of(e, e->cfg.root_polish != 0), (launch_trace_t<CVK>(S, d_rays, n, t_min, t_max, out, e->status.p, st), 0));
+    PHX_CV_RETURN(cv_of(e, e->cfg.root_polish != 0), (launch_trace_t<CVK>(e->device, S, d_rays, n, t_min, t_max, out, e->status.p, st)));
 }
 
 extern "C" {
@@ -1905,7 +1932,10 @@ int phx_trace_device(phx_engine* e, const float* d_rays, int64_t n, float t_min,
     PHX_CU(cudaSetDevice(e->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
     PHX_CU(cudaMemsetAsync(e->status.p, 0, sizeof(unsigned), st));
-    if (n > 0) launch_trace(e, d_rays, n, t_min, t_max, reinterpret_cast<float4*>(d_prd), st);
+    if (n > 0) {
+        const int rc = launch_trace(e, d_rays, n, t_min, t_max, reinterpret_cast<float4*>(d_prd), st);
+        if (rc) return rc;
+    }
     PHX_CU(cudaGetLastError());
     if (status) {
         PHX_CU(cudaMemcpyAsync(e->h_pinned, e->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));

