@@ -99,6 +99,7 @@ struct phx_engine {
     DevBuf<float4> leaf_sph;               // world bounding sphere per leaf (centre, radius)
     DevBuf<float4> global_q;               // plain global leaves (PhxScene.global_q)
     unsigned kind_mask = 0u;
+    bool plain = false;                    // every leaf is a plain global or of an inlined kind
     int num_global = 0;
     float cull[4] = { 0.f, 0.f, 0.f, 0.f };
     int num_node = 0, num_prim = 0, num_inst = 0, num_leaf = 0, bvh_depth = 0;
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(128) k_csg_scan(PhxCsgCtx csg, int root, float
 // reference's quad2 PRD (sysrap/squad.h:180-245): q0 normal.xyz (world, unnormalised), t;
 // q1 lposcost, 0, iindex<<16|identity, globalPrimIdx<<16|boundary (0xffffffff words: a miss)
 template <int CV>
-__global__ void __launch_bounds__(128, 3) k_trace_rays(PhxScene S, const float* rays, long long n, float t_min, float t_max,
+__global__ void __launch_bounds__(128, PHX_TRACE_MINB(CV)) k_trace_rays(PhxScene S, const float* rays, long long n, float t_min, float t_max,
                                                        float4* prd_out, unsigned* status)
 {
     __shared__ int2 queue[4 * 64];
@@ -1302,6 +1303,7 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
         std::vector<float> sph = bv.global_sphere;
         sph.insert(sph.end(), bv.leaf_sphere.begin(), bv.leaf_sphere.end());
         std::vector<float> gq(std::max<size_t>(1, bv.globals.size()) * 8, 0.f);
+        std::vector<char> plain_row(bv.globals.size(), 0);
         for (size_t g = 0; g < bv.globals.size(); g++) {
             const float* q = geo->node + 16 * (size_t)all[g].node_offset;
             const float* m = &inv[16 * (size_t)all[g].inst];
@@ -1313,10 +1315,17 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
             if (!plain) continue;
             memcpy(&gq[8 * g], q, 16);
             memcpy(&gq[8 * g + 4], &tc, 4);
+            plain_row[g] = 1;
         }
         if (geo->num_node < (1 << PHX_LEAF_KIND)) {
             e->kind_mask = 7u << PHX_LEAF_KIND;
-            for (phx_leaf& L : all) L.node_offset |= (int32_t)(prim_kind(geo, L.node_offset) << PHX_LEAF_KIND);
+            e->plain = !e->has_full;
+            for (size_t k = 0; k < all.size(); k++) {
+                const uint32_t kind = prim_kind(geo, all[k].node_offset);
+                const bool row = k < bv.globals.size() && plain_row[k] != 0;
+                e->plain = e->plain && (row || kind != PHX_KIND_ANY);
+                all[k].node_offset |= (int32_t)(kind << PHX_LEAF_KIND);
+            }
         }
         PHX_TRYCU(e->leaves.ensure(std::max<size_t>(1, all.size())));
         if (!all.empty()) PHX_TRYCU(cudaMemcpy(e->leaves.p, all.data(), all.size() * sizeof(phx_leaf), cudaMemcpyHostToDevice));
@@ -1429,6 +1438,12 @@ static int cv_of(const phx_engine* e, bool polish)
     return (polish ? PHX_CV_POLISH : 0) | (e->has_full ? PHX_CV_FULL : 0);
 }
 
+// the variant of the closest-hit kernels: the plain one where every leaf is of an inlined kind
+static int trace_cv_of(const phx_engine* e, bool polish)
+{
+    return e->plain && !polish ? PHX_CV_PLAIN : cv_of(e, polish);
+}
+
 // `return EXPR` with the compile-time constant CVK set to the runtime variant cv
 #define PHX_CV_RETURN(cv, EXPR)                               \
     switch (cv) {                                             \
@@ -1437,6 +1452,11 @@ static int cv_of(const phx_engine* e, bool polish)
         case 3: { constexpr int CVK = 3; return EXPR; }       \
         default: { constexpr int CVK = 0; return EXPR; }      \
     }
+
+// the same over the closest-hit kernels' variants
+#define PHX_TRACE_CV_RETURN(cv, EXPR)                                          \
+    if ((cv) == PHX_CV_PLAIN) { constexpr int CVK = PHX_CV_PLAIN; return EXPR; } \
+    PHX_CV_RETURN(cv, EXPR)
 
 template <int BLOCK, bool ADJ = false>
 static int launch_persistent_b(phx_engine* e, const PersistArgs& A, int cv, cudaStream_t st)
@@ -1492,12 +1512,14 @@ static long long wave_pool_for(const phx_engine* e, long long N, bool adj)
     }
     return std::max<long long>(1, std::min(std::min(N, pool), PHX_WAVE_POOL_MAX));
 }
-// Calls of at most this many photons skip the rounds: all their paths fit in the tail kernel's resident
-// lanes (56,832 of them), so a round's two launches only add to the latency of the longest path.
-// Detector events: 1,000 photons 140 us with two rounds, 118 without; 50k 242 / 217; 200k 469 / 475 (there
-// the coherent rounds pay again).
+// The rounds pay where many paths start coherently ahead of a hierarchy that the later bounces walk
+// divergently.  Calls of at most this many photons skip them: a round's two launches add more to the
+// longest path's latency than they save (detector events: 50k photons 217 us without rounds, 242 with
+// two; 200k 399 / 416; 500k 762 / 715).  So do calls on geometries without hierarchy leaves, whose
+// every bounce is coherent in the tail kernel's registers (1M torch photons in the sphere-in-box
+// 441-469 us, 556 with two rounds).
 #ifndef PHX_WAVE_SMALL
-#define PHX_WAVE_SMALL 65536
+#define PHX_WAVE_SMALL 262144
 #endif
 // calls of at most this many photons get their event-advanced RNG states in one coherent pass
 // ahead of the loop (24 B per photon of scratch); larger ones advance each state as it starts
@@ -1521,20 +1543,20 @@ static int wave_grid(K kernel, int dev, int* cache)
 template <int CV, bool ADJ = false>
 static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
 {
-    static int g_init[128] = {}, g_trace[128] = {}, g_shade[128] = {}, g_fill[128] = {}, g_tail[128] = {};
+    static int g_init[128] = {}, g_trace[128] = {}, g_shade[128] = {}, g_fill[128] = {}, g_tail_n[128] = {}, g_tail_w[128] = {};
+    constexpr bool TWO_TAILS = !ADJ && (CV & PHX_CV_PLAIN) != 0;
     const int dev = e->device;
     if (dev < 0 || dev >= 128) return phx_fail(-1, "device ordinal %d out of range", dev);
     int rc;
-    if ((rc = wave_grid(k_wave_init<CV, ADJ>, dev, g_init))) return rc;
-#if PHX_WAVE_TRACE_DF
-    if ((rc = wave_grid(k_wave_trace_df<CV>, dev, g_trace))) return rc;
-#else
+    if ((rc = wave_grid(k_wave_init<ADJ>, dev, g_init))) return rc;
     if ((rc = wave_grid(k_wave_trace<CV>, dev, g_trace))) return rc;
-#endif
-    if ((rc = wave_grid(k_wave_shade<CV, ADJ>, dev, g_shade))) return rc;
-    if ((rc = wave_grid(k_wave_fill<CV, ADJ>, dev, g_fill))) return rc;
-    if ((rc = wave_grid(k_wave_tail<CV, ADJ>, dev, g_tail))) return rc;
+    if ((rc = wave_grid(k_wave_shade<ADJ>, dev, g_shade))) return rc;
+    if ((rc = wave_grid(k_wave_fill<ADJ>, dev, g_fill))) return rc;
     const long long N = A.N;
+    const bool wide = TWO_TAILS && N >= PHX_TAIL_WIDE && !A.S.bvh_empty;
+    const auto tail_kernel = wide ? k_wave_tail<CV, ADJ, TWO_TAILS> : k_wave_tail<CV, ADJ, false>;
+    int* const g_tail = wide ? g_tail_w : g_tail_n;
+    if ((rc = wave_grid(tail_kernel, dev, g_tail))) return rc;
     const long long pool = wave_pool_for(e, N, ADJ);
     PHX_CU(e->wslot.ensure((size_t)pool)); PHX_CU(e->wprd.ensure((size_t)pool)); PHX_CU(e->wsidx.ensure((size_t)pool));
     PHX_CU(e->wact0.ensure((size_t)pool)); PHX_CU(e->wact1.ensure((size_t)pool)); PHX_CU(e->wcnt.ensure(4));
@@ -1561,28 +1583,24 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
     W.live_bits = nullptr;
     W.refill_idle = e->cfg.wave_refill;
     const unsigned gi = (unsigned)std::min<long long>(g_init[dev], (pool + 127) / 128);
-    k_wave_init<CV, ADJ><<<gi, 128, 0, st>>>(W);
+    k_wave_init<ADJ><<<gi, 128, 0, st>>>(W);
     W.live_bits = refill ? e->wlive.p : nullptr;
     PHX_CU(cudaGetLastError());
     int cur = 0;
     const int cfg_rounds = ADJ ? e->cfg.adj_wave_rounds : e->cfg.wave_rounds;
     if (cfg_rounds > 0 && !refill) {
-        const int rounds = !ADJ && N <= PHX_WAVE_SMALL ? 0 : cfg_rounds;
+        const int rounds = !ADJ && (N <= PHX_WAVE_SMALL || A.S.bvh_empty) ? 0 : cfg_rounds;
         // fixed schedule, no host read: wave_rounds rounds, then the tail kernel finishes whatever is
         // still live (it reads the count on the device; a grid-stride loop over any count), so the
         // whole call can be captured as a CUDA graph
         for (int r = 0; r < rounds; r++) {
             W.act_in = act[cur]; W.n_in = cnt[cur]; W.act_out = act[1 - cur]; W.n_out = cnt[1 - cur];
-#if PHX_WAVE_TRACE_DF
-            k_wave_trace_df<CV><<<(unsigned)g_trace[dev], 128, 0, st>>>(W);
-#else
             k_wave_trace<CV><<<(unsigned)g_trace[dev], 128, 0, st>>>(W);
-#endif
-            k_wave_shade<CV, ADJ><<<(unsigned)g_shade[dev], 128, 0, st>>>(W);
+            k_wave_shade<ADJ><<<(unsigned)g_shade[dev], 128, 0, st>>>(W);
             cur = 1 - cur;
         }
         W.act_in = act[cur]; W.n_in = cnt[cur];
-        k_wave_tail<CV, ADJ><<<(unsigned)g_tail[dev], 128, 0, st>>>(W);
+        tail_kernel<<<(unsigned)g_tail[dev], 128, 0, st>>>(W);
         PHX_CU(cudaGetLastError());
         e->last_rounds = rounds;
         e->last_tail = 1;
@@ -1598,15 +1616,11 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
     for (long long r = 0; r < max_rounds && !done;) {
         for (int k = 0; k < PHX_WAVE_ROUNDS; k++, r++) {
             W.act_in = act[cur]; W.n_in = cnt[cur]; W.act_out = act[1 - cur]; W.n_out = cnt[1 - cur];
-#if PHX_WAVE_TRACE_DF
-            k_wave_trace_df<CV><<<(unsigned)g_trace[dev], 128, 0, st>>>(W);
-#else
             k_wave_trace<CV><<<(unsigned)g_trace[dev], 128, 0, st>>>(W);
-#endif
-            k_wave_shade<CV, ADJ><<<(unsigned)g_shade[dev], 128, 0, st>>>(W);
+            k_wave_shade<ADJ><<<(unsigned)g_shade[dev], 128, 0, st>>>(W);
             nl += 2;
             if (filling) {
-                k_wave_fill<CV, ADJ><<<(unsigned)g_fill[dev], 128, 0, st>>>(W);
+                k_wave_fill<ADJ><<<(unsigned)g_fill[dev], 128, 0, st>>>(W);
                 k_word_scan<<<(unsigned)nlb, 256, 0, st>>>(e->wlive.p, nlw, e->wlive_off.p, e->wlive_blk.p);
                 k_block_scan<<<1, 1024, 0, st>>>(e->wlive_blk.p, (int)nlb, e->wlive_tot.p);
                 k_wave_act<<<(unsigned)((nlw + 255) / 256), 256, 0, st>>>(e->wlive.p, nlw, e->wlive_off.p, e->wlive_blk.p,
@@ -1636,7 +1650,7 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
         if (!done && queue_done && (long long)live <= e->cfg.wave_tail) {
             // few paths left and none queued: finish them in one kernel
             W.act_in = act[cur]; W.n_in = cnt[cur];
-            k_wave_tail<CV, ADJ><<<(unsigned)std::min<long long>(g_tail[dev], (live + 127) / 128), 128, 0, st>>>(W);
+            tail_kernel<<<(unsigned)std::min<long long>(g_tail[dev], (live + 127) / 128), 128, 0, st>>>(W);
             PHX_CU(cudaGetLastError());
             e->last_tail = 1;
             nl += 1;
@@ -1651,12 +1665,12 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
 template <bool ADJ = false>
 static int launch_wave_cv(phx_engine* e, const PersistArgs& A, int cv, cudaStream_t st)
 {
-    PHX_CV_RETURN(cv, (launch_wave_t<CVK, ADJ>(e, A, st)));
+    PHX_TRACE_CV_RETURN(cv, (launch_wave_t<CVK, ADJ>(e, A, st)));
 }
 
 static int launch_wave(phx_engine* e, const PersistArgs& A, cudaStream_t st)
 {
-    return launch_wave_cv(e, A, cv_of(e, e->cfg.root_polish != 0), st);
+    return launch_wave_cv(e, A, trace_cv_of(e, e->cfg.root_polish != 0), st);
 }
 
 template <int CV>
@@ -1699,7 +1713,7 @@ static int launch_trace_t(int device, const PhxScene& S, const float* d_rays, lo
 static int launch_trace(phx_engine* e, const float* d_rays, long long n, float t_min, float t_max, float4* out, cudaStream_t st)
 {
     const PhxScene S = scene_of(e, e->cfg.root_polish);
-    PHX_CV_RETURN(cv_of(e, e->cfg.root_polish != 0), (launch_trace_t<CVK>(e->device, S, d_rays, n, t_min, t_max, out, e->status.p, st)));
+    PHX_TRACE_CV_RETURN(trace_cv_of(e, e->cfg.root_polish != 0), (launch_trace_t<CVK>(e->device, S, d_rays, n, t_min, t_max, out, e->status.p, st)));
 }
 
 extern "C" {
@@ -2245,8 +2259,8 @@ int phx_adjoint_device(phx_engine* e, const float* d_gensteps, int32_t num_genst
     A.adj_pathwise = (flags & PHX_ADJ_PATHWISE) ? 1 : 0;
     A.adj_prim_node = e->prim_node_d.p;
     if (N > 0) {
-        const int cv = cv_of(e, false);
-        rc = e->cfg.kernel_mode == 2 ? launch_wave_cv<true>(e, A, cv, st) : launch_persistent_b<64, true>(e, A, cv, st);
+        rc = e->cfg.kernel_mode == 2 ? launch_wave_cv<true>(e, A, trace_cv_of(e, false), st)
+                                     : launch_persistent_b<64, true>(e, A, cv_of(e, false), st);
         if (rc) return rc;
     }
     PHX_CU(cudaMemcpyAsync(e->h_pinned, e->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));

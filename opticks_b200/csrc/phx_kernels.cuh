@@ -83,6 +83,8 @@ PHX_D void phx_test_leaf(const PhxScene& S, const int li, const int4 L, const fl
     } else if (kind == PHX_KIND_LEAF) {
         is = leaf_fast<PHX_CV_P(CV)>(S.csg.node, S.csg.itra, root, tmin, lo, ld);
         valid = is.w > tmin;
+    } else if constexpr ((CV & PHX_CV_PLAIN) != 0) {
+        return;
     } else {
         const PhxPrimHit h = intersect_prim_any<CV>(S.csg.node, S.csg.itra, S.csg.plan, root, tmin, lo, ld);
         is = h.is;
@@ -337,8 +339,8 @@ PHX_D bool phx_trace(const PhxScene& S, const float3& o, const float3& d, float 
 // coherent part never runs in the few lanes that happen to be free, rays the cull ball keeps out of
 // the hierarchy never hold a lane among walking ones, and a warp does not wait for its longest walk.
 // Same arithmetic and order per ray as phx_trace.  2^20 rays anywhere in the detector (a quarter of them
-// walk): 402 -> 160 us against one thread per ray; a 1M-photon event's third round, where every ray
-// walks, runs at 16.8 lanes instead of 12.7.
+// walk): 402 -> 160 us against one thread per ray (122 us in the plain variant, 16 warps per SM); a
+// 1M-photon event's third round, where every ray walks, runs at 16.8 lanes instead of 12.7.
 //   next()                       the warp's next window (its first ray; < 0: none left), warp-uniform
 //   tag(base, lane, tag)         the lane's ray of a window: false past the end
 //   load(tag, o, d, tmin)        its origin, direction and interval start

@@ -219,7 +219,7 @@ PHX_D void phx_event_rng(curandStateXORWOW& s, const PersistArgs& A, int gi, lon
     }
 }
 
-template <int CV, bool ADJ>
+template <bool ADJ>
 PHX_D void persist_start(PhxLane& L, const PersistArgs& A, long long idx, unsigned& status, PhxScore* sc,
                          const uint32_t* planes = nullptr)
 {
@@ -253,7 +253,7 @@ PHX_D void persist_start(PhxLane& L, const PersistArgs& A, long long idx, unsign
     L.ev = (int)ev;
 }
 
-template <int CV, bool ADJ>
+template <bool ADJ>
 PHX_D void persist_finish(PhxLane& L, const PersistArgs& A, const PhxScore* sc)
 {
     const long long idx = L.idx;
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(BLOCK, PHX_PERSIST_MINB(BLOCK)) k_sim_persiste
                 take = t;
             }
             if ((take >> lane) & 1u) {
-                persist_start<CV, ADJ>(L, A, wnext + __popc(take & lanes_below), status, sc);
+                persist_start<ADJ>(L, A, wnext + __popc(take & lanes_below), status, sc);
                 active = true;
             }
             wnext += __popc(take);
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(BLOCK, PHX_PERSIST_MINB(BLOCK)) k_sim_persiste
         if (!__any_sync(FULL, active)) break;
         for (int k = 0; k < regroup; k++) {
             if (active && persist_step<CV, ADJ>(L, A, status, sc)) {
-                persist_finish<CV, ADJ>(L, A, sc);
+                persist_finish<ADJ>(L, A, sc);
                 active = false;
             }
         }

@@ -47,11 +47,11 @@ struct WaveArgs {
     float4* score;            // ADJ: 8 float4 (the 32 score terms) per slot
     uint32_t* free_list;      // slots freed by this round's physics (refilled by k_wave_fill)
     unsigned* n_free;
-    unsigned* trace_ctr;      // rays of this round handed to warps (k_wave_trace_df); zeroed by the kernel before
+    unsigned* trace_ctr;      // rays of this round handed to warps (k_wave_trace); zeroed by the kernel before
     long long pool;           // slots (init only)
     uint32_t* live_bits;      // refill rounds: live slots as bits, turned into the next list in slot
                               // order by k_wave_act (null: live slots are appended to act_out)
-    int refill_idle;          // k_wave_trace_df: idle lanes a warp waits for before taking new rays
+    int refill_idle;          // k_wave_trace: idle lanes a warp waits for before taking new rays
 };
 
 // The slot's first 32 B sector (position, time, direction, q1.w) is all the closest-hit kernel
@@ -274,7 +274,7 @@ __global__ void k_wave_act(uint32_t* bits, long long nword, const uint32_t* word
 // Lanes in `need` take new photons from the queue until each has a path that can be traced
 // (photons that cannot take a first bounce are finished at once) or the queue is empty.
 // Returns true in the lanes that hold a live path.  Warp-collective.
-template <int CV, bool ADJ = false>
+template <bool ADJ = false>
 PHX_D bool wave_refill(PhxLane& L, const PersistArgs& A, bool need, unsigned& status, PhxScore* sc = nullptr,
                        const uint32_t* planes = nullptr)
 {
@@ -293,9 +293,9 @@ PHX_D bool wave_refill(PhxLane& L, const PersistArgs& A, bool need, unsigned& st
             if (idx >= A.N) {
                 need = false;
             } else {
-                persist_start<CV, ADJ>(L, A, idx, status, sc, planes);
+                persist_start<ADJ>(L, A, idx, status, sc, planes);
                 if (wave_can_trace(L, A)) { live = true; need = false; }
-                else persist_finish<CV, ADJ>(L, A, sc);
+                else persist_finish<ADJ>(L, A, sc);
             }
         }
     }
@@ -320,7 +320,7 @@ PHX_D const uint32_t* wave_jump_planes(const PersistArgs& A)
 #endif
 
 // fill the pool: every slot takes photons until it holds a live path or the queue is empty
-template <int CV, bool ADJ = false>
+template <bool ADJ = false>
 __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init(WaveArgs W)
 {
     unsigned status = 0;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < W.pool; base += stride) {
         const long long s = base + (threadIdx.x & 31);
-        const bool live = wave_refill<CV, ADJ>(L, W.A, s < W.pool, status, ADJ ? &score : nullptr, planes);
+        const bool live = wave_refill<ADJ>(L, W.A, s < W.pool, status, ADJ ? &score : nullptr, planes);
         wave_put(W, st, (uint32_t)s, L, live, true);
         if (ADJ && live) wave_store_score(W, (uint32_t)s, &score);
         wave_append(W, live, (uint32_t)s);
@@ -340,41 +340,23 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init
     if (status) atomicOr(W.A.status, status);
 }
 
-// closest hit of every live path (CSGOptiX/CSGOptiX7.cu:477-490: tmin by the last flag, optixTrace)
-// resident 128-thread blocks per SM asked of the compiler for the closest-hit kernel (caps its
-// registers: 3 -> 168 registers, 12 warps per SM; 4 -> 128 with spills, 12.7 ms against 12.3 for the
-// 10M-photon detector event)
-#ifndef PHX_WAVE_TRACE_MINB
-#define PHX_WAVE_TRACE_MINB 3
-#endif
-
-template <int CV>
-__global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace(WaveArgs W)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) { *W.n_out = 0u; *W.n_free = 0u; }   // the launches after this one append
-    const unsigned n = *W.n_in;
-    unsigned status = 0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)n; i += stride) {
-        const uint32_t s = W.act_in[i];
-        const PhxWaveSlot* o = W.slot + s;
-        const float4 q0 = o->q0, q1 = o->q1;
-        const float tmin = wave_tmin(W, q1);
-        const PhxPRD prd = phx_trace_step<CV>(W.A.S, make_float3(q0.x, q0.y, q0.z), make_float3(q1.x, q1.y, q1.z), tmin,
-                                                  W.A.C.tmax, status);
-        W.prd[s].nd = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
-        W.prd[s].lgi = make_uint4(__float_as_uint(prd.lposcost), prd.gp_bd, prd.ii_id, 0u);
-    }
-    if (status) atomicOr(W.A.status, status);
-}
+// Closest hit of every live path (CSGOptiX/CSGOptiX7.cu:477-490: tmin by the last flag, optixTrace).
+// Resident 128-thread blocks per SM asked of the compiler for the closest-hit and the tail kernel: both
+// wait for dependent loads, so warps in flight count for more than registers, as long as the cap
+// spills nothing hot.  The general evaluator's call keeps 217 registers: 3 blocks (168 registers); 4 cost
+// spills (10M-photon detector event 12.7 ms against 12.3).  Without it (PHX_CV_PLAIN) the closest-hit
+// kernel takes 123 registers and the tail kernel 149: 4 blocks each, and 5 of the tail kernel for large
+// calls (10M photons: tail at 4 blocks 9.76 ms, 5 blocks 9.36, 6 blocks 9.87).  Small calls are the
+// latency of single paths, which the 5-block cap's spills lengthen (50k photons 200 us at 4 blocks, 211
+// at 5; 1M Cerenkov photons 1,167 and 1,150).
+#define PHX_TRACE_MINB(cv) (((cv) & PHX_CV_PLAIN) != 0 ? 4 : 3)
+#define PHX_TAIL_MINB(cv, adj, wide) (!(adj) && ((cv) & PHX_CV_PLAIN) != 0 ? ((wide) ? 5 : 4) : 3)
+#define PHX_TAIL_WIDE (1LL << 19)       // photons of a call from which the 5-block tail kernel runs (with a hierarchy)
 
 // The closest-hit round as a stream of rays (phx_trace_stream): each warp takes the round's live slots 32
-// at a time, one atomic per window.  The PRDs are the same as the plain kernel's.
-#ifndef PHX_WAVE_TRACE_DF
-#define PHX_WAVE_TRACE_DF 1
-#endif
+// at a time, one atomic per window.  The PRDs are those of phx_trace.
 template <int CV>
-__global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(WaveArgs W)
+__global__ void __launch_bounds__(128, PHX_TRACE_MINB(CV)) k_wave_trace(WaveArgs W)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) { *W.n_out = 0u; *W.n_free = 0u; }   // the launches after this one append
     __shared__ int2 queue[4 * 64];
@@ -413,10 +395,8 @@ __global__ void __launch_bounds__(128, PHX_WAVE_TRACE_MINB) k_wave_trace_df(Wave
 // ends takes the next one of the list at once (one atomic per warp on the round's ray counter,
 // which the physics kernel left at zero), so the lanes of a warp do not wait for its longest path.
 // Photons, seq and hits are the same as the rounds would give.
-// (3 blocks of 128 per SM, 168 registers; with the closest-hit search inlined: 3 blocks 12.27 ms for the
-// 10M-photon detector event, 4 blocks 13.61, 5 blocks 13.36)
-template <int CV, bool ADJ = false>
-__global__ void __launch_bounds__(128, 3) k_wave_tail(WaveArgs W)
+template <int CV, bool ADJ = false, bool WIDE = false>
+__global__ void __launch_bounds__(128, PHX_TAIL_MINB(CV, ADJ, WIDE)) k_wave_tail(WaveArgs W)
 {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
@@ -453,7 +433,7 @@ __global__ void __launch_bounds__(128, 3) k_wave_tail(WaveArgs W)
         if (!__any_sync(FULL, has)) break;
         // persist_step ends a path within max_bounce steps
         if (has && persist_step<CV, ADJ>(L, W.A, status, ADJ ? &score : nullptr)) {
-            persist_finish<CV, ADJ>(L, W.A, ADJ ? &score : nullptr);
+            persist_finish<ADJ>(L, W.A, ADJ ? &score : nullptr);
             has = false;
         }
     }
@@ -473,7 +453,7 @@ __global__ void __launch_bounds__(128, 3) k_wave_tail(WaveArgs W)
 #endif
 
 // the physics of one path whose slot is in the warp's staging area; true when it goes on
-template <int CV, bool ADJ>
+template <bool ADJ>
 PHX_D bool wave_shade_path(const WaveArgs& W, const float4* st, uint32_t s, const float4 nd, const uint4 lgi, PhxLane& L,
                            PhxScore* sc, unsigned& status)
 {
@@ -502,12 +482,12 @@ PHX_D bool wave_shade_path(const WaveArgs& W, const float4* st, uint32_t s, cons
     }
     if (done) {
         L.idx = W.sidx[s];
-        persist_finish<CV, ADJ>(L, W.A, sc);
+        persist_finish<ADJ>(L, W.A, sc);
     }
     return !done;
 }
 
-template <int CV, bool ADJ = false>
+template <bool ADJ = false>
 __global__ void __launch_bounds__(128, ADJ ? PHX_WAVE_SHADE_ADJ_MINB : PHX_WAVE_SHADE_MINB) k_wave_shade(WaveArgs W)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0 && W.trace_ctr) *W.trace_ctr = 0u;   // for the next round's closest-hit kernel
@@ -528,7 +508,7 @@ __global__ void __launch_bounds__(128, ADJ ? PHX_WAVE_SHADE_ADJ_MINB : PHX_WAVE_
         uint4 lgi = make_uint4(0u, 0u, 0u, 0u);
         if (valid) { nd = W.prd[s].nd; lgi = W.prd[s].lgi; }     // in flight with the slot reads
         wave_gather(W, st, s, valid);
-        const bool live = valid && wave_shade_path<CV, ADJ>(W, st, s, nd, lgi, L, ADJ ? &score : nullptr, status);
+        const bool live = valid && wave_shade_path<ADJ>(W, st, s, nd, lgi, L, ADJ ? &score : nullptr, status);
         wave_put(W, st, s, L, live, false);
         if (ADJ && live) wave_store_score(W, s, &score);
         wave_append(W, live, s);
@@ -538,7 +518,7 @@ __global__ void __launch_bounds__(128, ADJ ? PHX_WAVE_SHADE_ADJ_MINB : PHX_WAVE_
 }
 
 // new photons from the queue into the slots freed this round (warp-coherent generation)
-template <int CV, bool ADJ = false>
+template <bool ADJ = false>
 __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_fill(WaveArgs W)
 {
     const unsigned n = *W.n_free;
@@ -558,7 +538,7 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_fill
         const long long i = base + (threadIdx.x & 31);
         const bool valid = i < (long long)n;
         const uint32_t s = valid ? W.free_list[i] : 0u;
-        const bool live = wave_refill<CV, ADJ>(L, W.A, valid, status, ADJ ? &score : nullptr, planes);
+        const bool live = wave_refill<ADJ>(L, W.A, valid, status, ADJ ? &score : nullptr, planes);
         wave_put(W, st, s, L, live, true);
         if (ADJ && live) wave_store_score(W, s, &score);
         wave_append(W, live, s);
