@@ -86,9 +86,10 @@ typedef struct {
     int32_t  wave_rounds;             /* wavefront schedule: n > 0 = n rounds and then the tail kernel
                                          for whatever is left, with no host read (a batched call is then
                                          captured as a CUDA graph, use_graph), when every photon of the
-                                         call is in flight at once (calls of up to 262,144 photons, and
-                                         calls on geometries whose leaves all span much of the scene,
-                                         go to the tail kernel at once); 0, or a call that refills slots =
+                                         call is in flight at once; where the first bounces need no
+                                         walk of the leaf hierarchy the starting kernel takes 2n of
+                                         them instead, and small calls, or calls on geometries without
+                                         a hierarchy, go to the tail kernel at once; 0, or a call that refills slots =
                                          the host reads the live count every few rounds and starts the
                                          tail kernel below wave_tail paths (2) */
     int64_t  wave_tail;               /* live paths at or below which the tail kernel finishes them

@@ -99,6 +99,7 @@ struct phx_engine {
     DevBuf<float4> leaf_sph;               // world bounding sphere per leaf (centre, radius)
     DevBuf<float4> global_q;               // plain global leaves (PhxScene.global_q)
     unsigned kind_mask = 0u;
+    bool plain_globals = false;            // every global leaf has a parameter row (PhxScene.global_q)
     bool plain = false;                    // every leaf is a plain global or of an inlined kind
     int num_global = 0;
     float cull[4] = { 0.f, 0.f, 0.f, 0.f };
@@ -1317,6 +1318,7 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
             memcpy(&gq[8 * g + 4], &tc, 4);
             plain_row[g] = 1;
         }
+        e->plain_globals = !bv.globals.empty() && std::count(plain_row.begin(), plain_row.end(), 1) == (long)bv.globals.size();
         if (geo->num_node < (1 << PHX_LEAF_KIND)) {
             e->kind_mask = 7u << PHX_LEAF_KIND;
             e->plain = !e->has_full;
@@ -1478,9 +1480,10 @@ static int launch_persistent(phx_engine* e, const PersistArgs& A, int block, cud
 
 // Wavefront form (phx_wave.cuh): fill a pool of paths, then rounds of trace + shade launches, then
 // the tail kernel for the paths still live.  When every photon of the call fits in the pool the
-// schedule is fixed (phx_config.wave_rounds rounds, 2 by default: the rounds that carry every path
-// through the scintillator and acrylic, where the wavefront's coherent launches pay; the longer,
-// divergent chains after them run faster in the tail kernel's registers than through the pool;
+// schedule is fixed (phx_config.wave_rounds rounds, 2 by default: the bounces that carry every path
+// through the scintillator and acrylic coherently, taken by the starting kernel where it can, see
+// PHX_WAVE_START_MIN; the longer, divergent chains after them run faster in the tail kernel's registers
+// than through the pool;
 // adjoint passes take phx_config.adj_wave_rounds, 12 by default), with no host read, so the call can
 // be captured into a graph.  Otherwise (refill, or wave_rounds 0) the
 // live count is read back every PHX_WAVE_ROUNDS rounds and the tail kernel starts below
@@ -1512,15 +1515,20 @@ static long long wave_pool_for(const phx_engine* e, long long N, bool adj)
     }
     return std::max<long long>(1, std::min(std::min(N, pool), PHX_WAVE_POOL_MAX));
 }
-// The rounds pay where many paths start coherently ahead of a hierarchy that the later bounces walk
+// Scenes without such a ball: the rounds pay where many paths start coherently ahead of a hierarchy that the later bounces walk
 // divergently.  Calls of at most this many photons skip them: a round's two launches add more to the
 // longest path's latency than they save (detector events: 50k photons 217 us without rounds, 242 with
 // two; 200k 399 / 416; 500k 762 / 715).  So do calls on geometries without hierarchy leaves, whose
 // every bounce is coherent in the tail kernel's registers (1M torch photons in the sphere-in-box
 // 441-469 us, 556 with two rounds).
-#ifndef PHX_WAVE_SMALL
 #define PHX_WAVE_SMALL 262144
-#endif
+// Where the scene has plain global leaves and a ball free of hierarchy leaves, calls of at least this
+// many photons take their first 2 wave_rounds bounces in the starting kernel (k_wave_start) instead of
+// in rounds.  Detector events, straight to the tail kernel / through k_wave_start: 10k photons 149 / 149 us,
+// 25k 171 / 162, 50k 202 / 190, 200k 402 / 373, 1M Cerenkov 1,158 / 1,000.  Below that the paths are better
+// spread over all warps from the start; without a hierarchy the tail kernel's refilled lanes are (1M
+// torch photons 397 / 437 us).
+#define PHX_WAVE_START_MIN 16384
 // calls of at most this many photons get their event-advanced RNG states in one coherent pass
 // ahead of the loop (24 B per photon of scratch); larger ones advance each state as it starts
 #define PHX_EV_RNG_MAX (1LL << 26)
@@ -1582,14 +1590,25 @@ static int launch_wave_t(phx_engine* e, const PersistArgs& A, cudaStream_t st)
     W.act_in = nullptr; W.n_in = nullptr; W.act_out = act[0]; W.n_out = cnt[0];
     W.live_bits = nullptr;
     W.refill_idle = e->cfg.wave_refill;
-    const unsigned gi = (unsigned)std::min<long long>(g_init[dev], (pool + 127) / 128);
-    k_wave_init<ADJ><<<gi, 128, 0, st>>>(W);
+    const int cfg_rounds = ADJ ? e->cfg.adj_wave_rounds : e->cfg.wave_rounds;
+    const bool fixed = cfg_rounds > 0 && !refill;
+    // the coherent first bounces: in k_wave_start where they need no hierarchy walk, else as rounds
+    const bool skip = !ADJ && (N <= PHX_WAVE_SMALL || A.S.bvh_empty);
+    const bool start = !ADJ && fixed && N >= PHX_WAVE_START_MIN && e->plain_globals && !A.S.bvh_empty && A.S.cull.w > 0.f;
+    if (start) {
+        static int g_start[2][128] = {};
+        const int pol = PHX_CV_P(CV) ? 1 : 0;
+        const auto start_kernel = k_wave_start<PHX_CV_P(CV)>;
+        if ((rc = wave_grid(start_kernel, dev, g_start[pol]))) return rc;
+        start_kernel<<<(unsigned)std::min<long long>(g_start[pol][dev], (pool + 127) / 128), 128, 0, st>>>(W, 2 * cfg_rounds);
+    } else {
+        k_wave_init<ADJ><<<(unsigned)std::min<long long>(g_init[dev], (pool + 127) / 128), 128, 0, st>>>(W);
+    }
     W.live_bits = refill ? e->wlive.p : nullptr;
     PHX_CU(cudaGetLastError());
     int cur = 0;
-    const int cfg_rounds = ADJ ? e->cfg.adj_wave_rounds : e->cfg.wave_rounds;
-    if (cfg_rounds > 0 && !refill) {
-        const int rounds = !ADJ && (N <= PHX_WAVE_SMALL || A.S.bvh_empty) ? 0 : cfg_rounds;
+    if (fixed) {
+        const int rounds = skip || start ? 0 : cfg_rounds;
         // fixed schedule, no host read: wave_rounds rounds, then the tail kernel finishes whatever is
         // still live (it reads the count on the device; a grid-stride loop over any count), so the
         // whole call can be captured as a CUDA graph

@@ -111,6 +111,25 @@ PHX_D void phx_test_range(const PhxScene& S, int first, int count, const float3&
     }
 }
 
+// Global leaf g if it has a parameter row (false: it has none)
+template <bool POLISH>
+PHX_D bool phx_test_plain_global(const PhxScene& S, int g, const float3& o, const float3& d, float tmin, PhxBest& B)
+{
+    const float4 q0 = __ldg(S.global_q + 2 * g);
+    const unsigned tc = __float_as_uint(__ldg(&S.global_q[2 * g + 1].x));
+    if (tc != PHX_CSG_SPHERE && tc != PHX_CSG_BOX3) return false;
+    float4 is;
+    bool valid;
+    if (tc == PHX_CSG_SPHERE) valid = leaf_sphere<POLISH>(is, q0, tmin, o, d);
+    else { is = leaf_box3(q0, tmin, o, d); valid = is.w > tmin; }
+    if (valid && is.w < B.t) {
+        B.t = is.w;
+        B.leaf = g;
+        B.n = make_float3(is.x, is.y, is.z);
+    }
+    return true;
+}
+
 // The global leaves, in order.  Plain spheres and boxes of the world solid (identity instance, no
 // node transform, no complement: the usual volumes around a detector) are solved from their parameter
 // row, without the instance transform, the node loads and the dispatch of the general leaf.
@@ -119,19 +138,7 @@ PHX_D void phx_test_globals(const PhxScene& S, const float3& o, const float3& d,
 {
 #pragma unroll 1
     for (int g = 0; g < S.num_global; g++) {
-        const float4 q0 = __ldg(S.global_q + 2 * g);
-        const unsigned tc = __float_as_uint(__ldg(&S.global_q[2 * g + 1].x));
-        if (tc == PHX_CSG_SPHERE || tc == PHX_CSG_BOX3) {
-            float4 is;
-            bool valid;
-            if (tc == PHX_CSG_SPHERE) valid = leaf_sphere<PHX_CV_P(CV)>(is, q0, tmin, o, d);
-            else { is = leaf_box3(q0, tmin, o, d); valid = is.w > tmin; }
-            if (valid && is.w < B.t) {
-                B.t = is.w;
-                B.leaf = g;
-                B.n = make_float3(is.x, is.y, is.z);
-            }
-        } else {
+        if (!phx_test_plain_global<PHX_CV_P(CV)>(S, g, o, d, tmin, B)) {
             const int4 L = __ldg(reinterpret_cast<const int4*>(S.leaves + g));
             if (phx_ball_overlaps(__ldg(S.leaf_sph + g), o, d, tmin, B.t)) phx_test_leaf<CV>(S, g, L, o, d, tmin, B, status);
         }

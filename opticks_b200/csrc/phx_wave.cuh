@@ -340,6 +340,58 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init
     if (status) atomicOr(W.A.status, status);
 }
 
+// Fill the pool and take each path through its first bounces, as long as they need no walk of the
+// hierarchy: the closest hit lies on a plain global leaf and the cull ball holds the segment (the
+// scintillator, acrylic and inner water of the detector).  These bounces are coherent (the lanes hold
+// consecutive photons of a genstep) and short, so they run here in registers; as wavefront rounds each
+// would write and read the 128 B path and its 32 B PRD.  A path that must walk, or has taken `bounces`,
+// goes to its slot for the tail kernel.  For scenes whose globals are all plain.
+// Bound by the physics step's issue and the RNG state reads: 10M-photon detector event 10.2 -> 8.1 ms with
+// two bounces here instead of two rounds, 7.8 with four (one 9.5, three 7.8, six 7.9).  4 blocks per SM:
+// 96 registers without spills (5 blocks 8.11 ms, 6 blocks 8.24, 7 blocks 8.52, against 8.08).
+#define PHX_WAVE_START_MINB 4
+template <bool POLISH>
+__global__ void __launch_bounds__(128, PHX_WAVE_START_MINB) k_wave_start(WaveArgs W, int bounces)
+{
+    const unsigned FULL = 0xffffffffu;
+    const PhxScene& S = W.A.S;
+    unsigned status = 0;
+    PhxLane L;
+    float4* st = wave_stage_area();
+    const uint32_t* planes = wave_jump_planes(W.A);
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < W.pool; base += stride) {
+        const long long s = base + (threadIdx.x & 31);
+        bool live = wave_refill<false>(L, W.A, s < W.pool, status, nullptr, planes);
+        bool go = live;
+        for (int b = 0; b < bounces && __any_sync(FULL, go); b++) {
+            if (!go) continue;
+            const float tmin = (L.p.obf & W.A.C.eps0_mask) ? W.A.C.tmin0 : W.A.C.tmin;
+            PhxBest B;
+            B.t = W.A.C.tmax; B.leaf = -1; B.n = make_float3(0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (int g = 0; g < S.num_global; g++) phx_test_plain_global<POLISH>(S, g, L.p.pos, L.p.mom, tmin, B);
+            if (!S.bvh_empty && !phx_culled(S, L.p.pos, L.p.mom, tmin, B.t)) { go = false; continue; }
+            PhxPRD prd;
+            phx_best_prd(S, B, L.p.pos, L.p.mom, prd);
+            bool done = true;
+            if (prd.boundary() != 0xffffu) {
+                const int command = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
+                L.bounce++;
+                seq_add_nibble(L.seqhis, L.seqbnd, (unsigned)L.bounce, L.p.flag(), L.p.boundary());
+                done = command == PHX_BREAK || !wave_can_trace(L, W.A);
+            }
+            if (done) {
+                persist_finish<false>(L, W.A, nullptr);
+                live = go = false;
+            }
+        }
+        wave_put(W, st, (uint32_t)s, L, live, true);
+        wave_append(W, live, (uint32_t)s);
+    }
+    if (status) atomicOr(W.A.status, status);
+}
+
 // Closest hit of every live path (CSGOptiX/CSGOptiX7.cu:477-490: tmin by the last flag, optixTrace).
 // Resident 128-thread blocks per SM asked of the compiler for the closest-hit and the tail kernel: both
 // wait for dependent loads, so warps in flight count for more than registers, as long as the cap
