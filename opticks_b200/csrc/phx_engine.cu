@@ -1920,7 +1920,7 @@ int phx_csg_scan_device(phx_engine* e, int32_t prim, float t_min, const float* d
     if (prim < 0 || prim >= e->num_prim) return phx_fail(-1, "phx_csg_scan_device: prim %d out of range", prim);
     PHX_CU(cudaSetDevice(e->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : e->stream;
-    PHX_CU(cudaMemsetAsync(e->status.p, 0, sizeof(unsigned), st));
+    // (a scan reports no status; every call that does clears the word first)
     const PhxCsgCtx csg = e->csg;
     if (n > 0) {
         float4* out = reinterpret_cast<float4*>(d_isect);
