@@ -112,46 +112,57 @@ PHX_STEPFN_T PhxPRD phx_trace_step(const PhxScene S, const float3 o, const float
 }
 
 // the PRD normal is normalised here (CSGOptiX/CSGOptiX7.cu:491-498) as part of the shared step
-#ifndef PHX_PROP_IO
-#define PHX_PROP_IO 1
-#endif
-#if PHX_PROP_IO
-// The photon and its RNG state go in and come back by value: the out-of-line step then takes no
-// address of the caller's copies, which stay in registers (by reference they live in local
-// memory for the whole caller).  Every caller shares this one compiled step.
+// What the step reads and writes of a path goes in and comes back by value: the out-of-line step then
+// takes no address of the caller's copies, which stay in registers (by reference they live in local
+// memory for the whole caller).  The argument itself passes through local memory, so it holds the 22
+// words the step needs: no photon index, and of the RNG state the five XORWOW words and the counter
+// (cuRAND's Box-Muller fields are never used here).  Every caller shares this one compiled step.
 struct PhxStepIO {
-    PhxPhoton p;
-    curandStateXORWOW rng;
-    unsigned status;
-    int command;
+    float3 pos; float time;
+    float3 mom; float wavelength;
+    float3 pol;
+    unsigned obf, identity, flagmask, hitcount_iindex;
+    unsigned d, v[5];
+    unsigned status_command;      // status bits, the command in bit 31
 };
-PHX_STEPFN_P PhxStepIO phx_propagate_io(PhxStepIO io, PhxPRD prd, const PhxProps P)
+PHX_STEPFN_P PhxStepIO phx_propagate_io(const PhxStepIO in, PhxPRD prd, const PhxProps P)
 {
+    PhxPhoton p;
+    p.pos = in.pos; p.time = in.time; p.mom = in.mom; p.wavelength = in.wavelength; p.pol = in.pol;
+    p.obf = in.obf; p.identity = in.identity; p.flagmask = in.flagmask; p.hitcount_iindex = in.hitcount_iindex; p.index = 0u;
+    curandStateXORWOW rng;
+    rng.d = in.d;
+    rng.v[0] = in.v[0]; rng.v[1] = in.v[1]; rng.v[2] = in.v[2]; rng.v[3] = in.v[3]; rng.v[4] = in.v[4];
+    rng.boxmuller_flag = 0; rng.boxmuller_flag_double = 0; rng.boxmuller_extra = 0.f; rng.boxmuller_extra_double = 0.0;
+    unsigned status = 0u;
     prd.normal = normalize(prd.normal);
-    io.command = propagate<false>(io.p, io.rng, prd, P, io.status, nullptr);
-    return io;
+    const int command = propagate<false>(p, rng, prd, P, status, nullptr);
+    PhxStepIO out;
+    out.pos = p.pos; out.time = p.time; out.mom = p.mom; out.wavelength = p.wavelength; out.pol = p.pol;
+    out.obf = p.obf; out.identity = p.identity; out.flagmask = p.flagmask; out.hitcount_iindex = p.hitcount_iindex;
+    out.d = rng.d;
+    out.v[0] = rng.v[0]; out.v[1] = rng.v[1]; out.v[2] = rng.v[2]; out.v[3] = rng.v[3]; out.v[4] = rng.v[4];
+    out.status_command = status | (command == PHX_BREAK ? 0x80000000u : 0u);
+    return out;
 }
 
-PHX_D int phx_propagate_step(PhxPhoton& p, curandStateXORWOW& rng, PhxPRD prd, const PhxProps& P, unsigned& status)
+// true when the path ends (PHX_BREAK)
+PHX_D bool phx_propagate_step(PhxPhoton& p, curandStateXORWOW& rng, const PhxPRD& prd, const PhxProps& P, unsigned& status)
 {
     PhxStepIO io;
-    io.p = p;
-    io.rng = rng;
-    io.status = 0u;
-    io.command = 0;
+    io.pos = p.pos; io.time = p.time; io.mom = p.mom; io.wavelength = p.wavelength; io.pol = p.pol;
+    io.obf = p.obf; io.identity = p.identity; io.flagmask = p.flagmask; io.hitcount_iindex = p.hitcount_iindex;
+    io.d = rng.d;
+    io.v[0] = rng.v[0]; io.v[1] = rng.v[1]; io.v[2] = rng.v[2]; io.v[3] = rng.v[3]; io.v[4] = rng.v[4];
+    io.status_command = 0u;
     io = phx_propagate_io(io, prd, P);
-    p = io.p;
-    rng = io.rng;
-    status |= io.status;
-    return io.command;
+    p.pos = io.pos; p.time = io.time; p.mom = io.mom; p.wavelength = io.wavelength; p.pol = io.pol;
+    p.obf = io.obf; p.identity = io.identity; p.flagmask = io.flagmask; p.hitcount_iindex = io.hitcount_iindex;
+    rng.d = io.d;
+    rng.v[0] = io.v[0]; rng.v[1] = io.v[1]; rng.v[2] = io.v[2]; rng.v[3] = io.v[3]; rng.v[4] = io.v[4];
+    status |= io.status_command & 0x7fffffffu;
+    return (io.status_command & 0x80000000u) != 0u;
 }
-#else
-PHX_STEPFN_P int phx_propagate_step(PhxPhoton& p, curandStateXORWOW& rng, PhxPRD prd, const PhxProps P, unsigned& status)
-{
-    prd.normal = normalize(prd.normal);
-    return propagate<false>(p, rng, prd, P, status, nullptr);
-}
-#endif
 
 // The adjoint's physics step out of line, for the loops that hold a path over many bounces: compiled
 // apart from the closest-hit search, its roundings are those of the wavefront's physics kernel (the
@@ -297,15 +308,12 @@ PHX_D bool persist_step(PhxLane& L, const PersistArgs& A, unsigned& status, PhxS
     if (ADJ) phx_trace<CV>(A.S, L.p.pos, L.p.mom, tmin, A.C.tmax, prd, status);
     else prd = phx_trace_step<CV>(A.S, L.p.pos, L.p.mom, tmin, A.C.tmax, status);
     if (prd.boundary() == 0xffffu) return true;
-    int command;
-    if (ADJ) {
-        command = propagate_adj(L.p, L.rng, prd, A.P, status, sc);
-    } else {
-        command = phx_propagate_step(L.p, L.rng, prd, A.P, status);
-    }
+    bool ends;
+    if (ADJ) ends = propagate_adj(L.p, L.rng, prd, A.P, status, sc) == PHX_BREAK;
+    else ends = phx_propagate_step(L.p, L.rng, prd, A.P, status);
     L.bounce++;
     seq_add_nibble(L.seqhis, L.seqbnd, (unsigned)L.bounce, L.p.flag(), L.p.boundary());
-    return command == PHX_BREAK;
+    return ends;
 }
 
 // Minimum resident warps per SM asked of the compiler (caps registers per thread); 0 leaves the

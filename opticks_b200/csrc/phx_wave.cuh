@@ -376,10 +376,10 @@ __global__ void __launch_bounds__(128, PHX_WAVE_START_MINB) k_wave_start(WaveArg
             phx_best_prd(S, B, L.p.pos, L.p.mom, prd);
             bool done = true;
             if (prd.boundary() != 0xffffu) {
-                const int command = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
+                const bool ends = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
                 L.bounce++;
                 seq_add_nibble(L.seqhis, L.seqbnd, (unsigned)L.bounce, L.p.flag(), L.p.boundary());
-                done = command == PHX_BREAK || !wave_can_trace(L, W.A);
+                done = ends || !wave_can_trace(L, W.A);
             }
             if (done) {
                 persist_finish<false>(L, W.A, nullptr);
@@ -521,16 +521,16 @@ PHX_D bool wave_shade_path(const WaveArgs& W, const float4* st, uint32_t s, cons
     prd.ii_id = lgi.z;
     bool done = true;
     if (prd.boundary() != 0xffffu) {
-        int command;
+        bool ends;
         if (ADJ) {
             prd.normal = fx_unit(prd.normal);
-            command = propagate<true>(L.p, L.rng, prd, W.A.P, status, sc);
+            ends = propagate<true>(L.p, L.rng, prd, W.A.P, status, sc) == PHX_BREAK;
         } else {
-            command = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
+            ends = phx_propagate_step(L.p, L.rng, prd, W.A.P, status);
         }
         L.bounce++;
         seq_add_nibble(L.seqhis, L.seqbnd, (unsigned)L.bounce, L.p.flag(), L.p.boundary());
-        done = command == PHX_BREAK || !wave_can_trace(L, W.A);
+        done = ends || !wave_can_trace(L, W.A);
     }
     if (done) {
         L.idx = W.sidx[s];
