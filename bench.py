@@ -58,14 +58,13 @@ BYTES_PER_PHOTON_FIXED = 48 + 64 + 32
 SAMPLE_PER_GENSTEP = 30        # CPU sample: this many photons of every genstep of the event
 # DRAM bytes (read + write) of all kernels of one simulate call of this 10M-photon event, from a
 # one-pass ncu capture of the bench's own launches (profiles/launches_dram_wavefront_detector_10M.md)
-DRAM_TRAFFIC = {"bytes_per_call": 12.723e9, "photons": 10_000_000,
-                "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum summed over the 12 launches of one "
+DRAM_TRAFFIC = {"bytes_per_call": 4.377e9, "photons": 10_000_000,
+                "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum summed over the 6 launches of one "
                           "10M-photon simulate call of this workload (profiles/launches_dram_wavefront_detector_10M.md)"}
-# issue figures of the dominant kernel (k_wave_tail, 68 % of the step) from its ncu --set full
-# capture (profiles/k_wave_tail_detector_2M_ncu_full.md)
-ISSUE = {"kernel": "k_wave_tail", "share_of_step": 0.68, "issue_active": 0.387, "threads_per_warp_inst": 9.71,
-         "warps_active": 0.184, "lane_issue_frac": 0.387 * 9.71 / 32,
-         "source": "profiles/k_wave_tail_detector_2M_ncu_full.md"}
+# issue figures of the dominant kernel (k_wave_tail, 60 % of the step) from its ncu capture
+ISSUE = {"kernel": "k_wave_tail", "share_of_step": 0.60, "issue_active": 0.53, "threads_per_warp_inst": 9.30,
+         "warps_active": 0.287, "lane_issue_frac": 0.53 * 9.30 / 32,
+         "source": "profiles/k_wave_start_tail_detector_1M.md"}
 
 
 def load_peaks():
@@ -757,8 +756,8 @@ def main():
                 "config": {"workload": "detector-17612pmt-scint-10M", "gensteps": len(gs), "photons_per_genstep": int(ppg),
                            "photons_per_step": N, "outputs": "photon+seq+hits(SD)+sensor counts",
                            "l2": "inputs larger than L2 (RNG states 240 MB read + 960 MB written per step)",
-                           "kernel": (f"wavefront: closest-hit and physics kernels over every photon of the event "
-                                      f"in flight, {rounds} rounds per step, then the tail kernel" if mode == 2 else
+                           "kernel": (f"wavefront: every photon of the event in flight, first bounces in the starting "
+                                      f"kernel, {rounds} rounds per step, then the tail kernel" if mode == 2 else
                                       "persistent work queue, block 64, refill every bounce"),
                            "parallelism": f"{world} independent event streams" if world > 1 else "1 GPU"},
                 "gpu_launches": launches,
@@ -768,7 +767,7 @@ def main():
                              "traffic_source": DRAM_TRAFFIC["source"] if mode == 2 else None,
                              "issue": ISSUE if mode == 2 else None,
                              "kernel_ms": k_ms,
-                             "kernel": ("k_wave_init + 2 k_wave_trace_df/k_wave_shade rounds + k_wave_tail (whole simulate launch sequence)"
+                             "kernel": ("k_wave_start (generation and first bounces) + k_wave_tail (whole simulate launch sequence)"
                                         if mode == 2 else "k_sim_persistent (whole simulate launch sequence)"),
                              "bytes_per_photon": bytes_per_photon, "peak_kind": f"{peak_kind} hbm_gbs",
                              "note": "issue/latency-bound divergent ray tracing + physics; HBM roof far from binding"},

@@ -4,22 +4,24 @@
 // The one-kernel loop (phx_persist.cuh) keeps every path in registers, so the whole bounce —
 // traversal, CSG, generation, propagate, bookkeeping — is compiled as one function whose register
 // count (about 200) leaves ten warps per SM to hide the latency of the traversal's dependent
-// loads.  Here a round is two launches:
-//   k_wave_trace  reads ray origin/direction of every live path, runs phx_trace and writes the PRD
-//                 (a lean kernel: 168 registers, 12 warps per SM, against about 200 and 10)
+// loads.  Here a call is
+//   k_wave_start  generates the photons and takes their first bounces where no hierarchy walk is needed
+//                 (else k_wave_init generates them, and rounds of two launches follow:
+//   k_wave_trace  reads ray origin/direction of every live path and writes its PRD
 //   k_wave_shade  reads the path and its PRD, runs propagate / seq nibble / finish exactly as the
 //                 one-kernel loop does, and appends live slots to the next round's list and
 //                 finished slots to a free list
 //   k_wave_fill   (only when the event has more photons than slots) gives every free slot the next
 //                 photon from the queue: whole warps take consecutive photons of one genstep, so
-//                 generation runs coherently instead of in the few lanes that just finished
+//                 generation runs coherently instead of in the few lanes that just finished)
+//   k_wave_tail   runs the paths still live to their end
 // Path state is 128 B per slot (sphoton, the XORWOW words, bounce, event, seqhis/seqbnd) plus a
 // 32 B PRD; the extra HBM traffic is about 0.4 KB per bounce against microseconds of traversal.
 // Every photon consumes its random numbers in the same order as in the one-kernel loop, so
 // photons, seq and hits are bit-identical to it.
 //
-// The host drives rounds until the live count reaches zero (read back every few rounds); the
-// number of rounds is bounded by (N / pool + 1) * (max_bounce + 1).
+// A fixed number of rounds needs no host read; otherwise the host drives rounds until few paths are live
+// (read back every few rounds), and their number is bounded by (N / pool + 1) * (max_bounce + 1).
 #pragma once
 #include "phx_persist.cuh"
 
