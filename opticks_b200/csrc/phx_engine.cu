@@ -63,6 +63,20 @@ struct DevBuf {
     void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
 };
 
+// Host arrays to the device on stream st, which is waited for: the copy has landed on return.  (A copy
+// of pageable memory on the default stream may return before its last transfer, and the engine's own
+// stream is not ordered behind the default stream.)
+static cudaError_t phx_upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+static cudaError_t phx_upload_rows(cudaArray_t dst, const void* src, size_t row_bytes, size_t rows, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemcpy2DToArrayAsync(dst, 0, 0, src, row_bytes, row_bytes, rows, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 #include "phx_merge.cuh"
 
 // scratch of the hit merge (grow-only, per engine)
@@ -992,11 +1006,11 @@ extern "C" int phx_planck_icdf(float* out, int n)
     return 0;
 }
 
-static int make_texture_f4(cudaArray_t& arr, cudaTextureObject_t& tex, const float* data, int width, int height)
+static int make_texture_f4(cudaArray_t& arr, cudaTextureObject_t& tex, const float* data, int width, int height, cudaStream_t st)
 {
     cudaChannelFormatDesc ch = cudaCreateChannelDesc<float4>();
     PHX_CU(cudaMallocArray(&arr, &ch, width, height));
-    PHX_CU(cudaMemcpy2DToArray(arr, 0, 0, data, width * sizeof(float4), width * sizeof(float4), height, cudaMemcpyHostToDevice));
+    PHX_CU(phx_upload_rows(arr, data, width * sizeof(float4), height, st));
     cudaResourceDesc rd;
     memset(&rd, 0, sizeof(rd));
     rd.resType = cudaResourceTypeArray;
@@ -1012,11 +1026,11 @@ static int make_texture_f4(cudaArray_t& arr, cudaTextureObject_t& tex, const flo
     return 0;
 }
 
-static int make_texture_f1(cudaArray_t& arr, cudaTextureObject_t& tex, const float* data, int width, int height)
+static int make_texture_f1(cudaArray_t& arr, cudaTextureObject_t& tex, const float* data, int width, int height, cudaStream_t st)
 {
     cudaChannelFormatDesc ch = cudaCreateChannelDesc<float>();
     PHX_CU(cudaMallocArray(&arr, &ch, width, height));
-    PHX_CU(cudaMemcpy2DToArray(arr, 0, 0, data, width * sizeof(float), width * sizeof(float), height, cudaMemcpyHostToDevice));
+    PHX_CU(phx_upload_rows(arr, data, width * sizeof(float), height, st));
     cudaResourceDesc rd;
     memset(&rd, 0, sizeof(rd));
     rd.resType = cudaResourceTypeArray;
@@ -1207,11 +1221,11 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     e->num_prim = geo->num_prim;
     e->num_inst = geo->num_inst;
     PHX_TRYCU(e->node.ensure((size_t)geo->num_node * 4));
-    PHX_TRYCU(cudaMemcpy(e->node.p, geo->node, (size_t)geo->num_node * 64, cudaMemcpyHostToDevice));
+    PHX_TRYCU(phx_upload(e->node.p, geo->node, (size_t)geo->num_node * 64, e->stream));
     PHX_TRYCU(e->itra.ensure((size_t)std::max(1, geo->num_itra) * 4));
-    if (geo->num_itra > 0) PHX_TRYCU(cudaMemcpy(e->itra.p, geo->itra, (size_t)geo->num_itra * 64, cudaMemcpyHostToDevice));
+    if (geo->num_itra > 0) PHX_TRYCU(phx_upload(e->itra.p, geo->itra, (size_t)geo->num_itra * 64, e->stream));
     PHX_TRYCU(e->plan.ensure((size_t)std::max(1, geo->num_plan)));
-    if (geo->num_plan > 0) PHX_TRYCU(cudaMemcpy(e->plan.p, geo->plan, (size_t)geo->num_plan * 16, cudaMemcpyHostToDevice));
+    if (geo->num_plan > 0) PHX_TRYCU(phx_upload(e->plan.p, geo->plan, (size_t)geo->num_plan * 16, e->stream));
     e->csg.node = e->node.p;
     e->csg.itra = e->itra.p;
     e->csg.plan = e->plan.p;
@@ -1228,7 +1242,7 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     }
     if (geo->num_prim > 0) {   // root node per prim on the device (the adjoint's probe intersections)
         PHX_TRYCU(e->prim_node_d.ensure((size_t)geo->num_prim));
-        PHX_TRYCU(cudaMemcpy(e->prim_node_d.p, e->prim_node_offset.data(), sizeof(int) * (size_t)geo->num_prim, cudaMemcpyHostToDevice));
+        PHX_TRYCU(phx_upload(e->prim_node_d.p, e->prim_node_offset.data(), sizeof(int) * (size_t)geo->num_prim, e->stream));
     }
     for (int i = 0; i < geo->num_node && !e->has_full; i++) {
         uint32_t tc;
@@ -1293,7 +1307,7 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     e->bvh_depth = bv.max_depth;
     if (3 * (bv.max_depth + 1) + 4 > PHX_BVH_STACK) { phx_destroy(e); return phx_fail(-1, "phx_create: BVH depth %d exceeds traversal stack", bv.max_depth); }
     PHX_TRYCU(e->bvh.ensure(std::max<size_t>(1, bv.nodes.size())));
-    if (!bv.nodes.empty()) PHX_TRYCU(cudaMemcpy(e->bvh.p, bv.nodes.data(), bv.nodes.size() * sizeof(phx_bvh4_node), cudaMemcpyHostToDevice));
+    if (!bv.nodes.empty()) PHX_TRYCU(phx_upload(e->bvh.p, bv.nodes.data(), bv.nodes.size() * sizeof(phx_bvh4_node), e->stream));
     e->num_global = (int)bv.globals.size();
     memcpy(e->cull, bv.cull, sizeof(e->cull));
     {
@@ -1330,14 +1344,14 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
             }
         }
         PHX_TRYCU(e->leaves.ensure(std::max<size_t>(1, all.size())));
-        if (!all.empty()) PHX_TRYCU(cudaMemcpy(e->leaves.p, all.data(), all.size() * sizeof(phx_leaf), cudaMemcpyHostToDevice));
+        if (!all.empty()) PHX_TRYCU(phx_upload(e->leaves.p, all.data(), all.size() * sizeof(phx_leaf), e->stream));
         PHX_TRYCU(e->leaf_sph.ensure(std::max<size_t>(1, sph.size() / 4)));
-        if (!sph.empty()) PHX_TRYCU(cudaMemcpy(e->leaf_sph.p, sph.data(), sph.size() * sizeof(float), cudaMemcpyHostToDevice));
+        if (!sph.empty()) PHX_TRYCU(phx_upload(e->leaf_sph.p, sph.data(), sph.size() * sizeof(float), e->stream));
         PHX_TRYCU(e->global_q.ensure(gq.size() / 4));
-        PHX_TRYCU(cudaMemcpy(e->global_q.p, gq.data(), gq.size() * sizeof(float), cudaMemcpyHostToDevice));
+        PHX_TRYCU(phx_upload(e->global_q.p, gq.data(), gq.size() * sizeof(float), e->stream));
     }
     PHX_TRYCU(e->inst_inv.ensure(inv.size() / 4));
-    PHX_TRYCU(cudaMemcpy(e->inst_inv.p, inv.data(), inv.size() * sizeof(float), cudaMemcpyHostToDevice));
+    PHX_TRYCU(phx_upload(e->inst_inv.p, inv.data(), inv.size() * sizeof(float), e->stream));
 
     // ---- physics
     if (!phys->bnd || phys->num_bnd <= 0 || phys->num_wl <= 1 || !phys->optical) { phx_destroy(e); return phx_fail(-1, "phx_create: bnd/optical missing"); }
@@ -1348,30 +1362,30 @@ int phx_create(const phx_geometry* geo, const phx_physics* phys, const phx_confi
     e->nm0 = phys->wl_low;
     e->nms = phys->wl_step;
     e->bnd_host.assign(phys->bnd, phys->bnd + (size_t)phys->num_bnd * 8 * phys->num_wl * 4);
-    PHX_TRY(make_texture_f4(e->bnd_arr, e->bnd_tex, phys->bnd, (int)e->nx, (int)e->ny));
+    PHX_TRY(make_texture_f4(e->bnd_arr, e->bnd_tex, phys->bnd, (int)e->nx, (int)e->ny, e->stream));
     PHX_TRYCU(e->optical.ensure((size_t)phys->num_bnd * 4));
-    PHX_TRYCU(cudaMemcpy(e->optical.p, phys->optical, (size_t)phys->num_bnd * 4 * 16, cudaMemcpyHostToDevice));
+    PHX_TRYCU(phx_upload(e->optical.p, phys->optical, (size_t)phys->num_bnd * 4 * 16, e->stream));
     e->optical_host.assign(phys->optical, phys->optical + (size_t)phys->num_bnd * 16);
     if (phys->icdf && phys->icdf_width > 1 && phys->icdf_layers > 0) {
         e->hd_factor = (unsigned)phys->hd_factor;
-        PHX_TRY(make_texture_f1(e->icdf_arr, e->icdf_tex, phys->icdf, phys->icdf_width, phys->icdf_layers));
+        PHX_TRY(make_texture_f1(e->icdf_arr, e->icdf_tex, phys->icdf, phys->icdf_width, phys->icdf_layers, e->stream));
     } else {
         e->hd_factor = 0xffffffffu;  // no scintillator table : reemission wavelength 0
         float dummy[4] = { 0.f, 0.f, 0.f, 0.f };
-        PHX_TRY(make_texture_f1(e->icdf_arr, e->icdf_tex, dummy, 2, 2));
+        PHX_TRY(make_texture_f1(e->icdf_arr, e->icdf_tex, dummy, 2, 2, e->stream));
     }
     {
         // black-body wavelengths for torch photons without a wavelength (QPlanck)
         float table[PHX_PLANCK_N];
         phx_planck_icdf(table, PHX_PLANCK_N);
-        PHX_TRY(make_texture_f1(e->planck_arr, e->planck_tex, table, PHX_PLANCK_N, 1));
+        PHX_TRY(make_texture_f1(e->planck_arr, e->planck_tex, table, PHX_PLANCK_N, 1, e->stream));
     }
     // ---- rng + small buffers
     {
         const std::vector<uint32_t> pw = phx_jump_powers(e->cfg.skipahead_event_offset);
         DevBuf<uint32_t> pow;
         PHX_TRYCU(pow.ensure(pw.size()));
-        cudaError_t ce = cudaMemcpy(pow.p, pw.data(), pw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+        cudaError_t ce = phx_upload(pow.p, pw.data(), pw.size() * sizeof(uint32_t), e->stream);
         if (ce == cudaSuccess) ce = e->jump_digit.ensure((size_t)PHX_JUMP_DIGITS * 15 * PHX_JUMP_NIBW);
         if (ce == cudaSuccess) {
             k_jump_digits<<<PHX_JUMP_DIGITS * 15, PHX_JUMP_THREADS, 0, e->stream>>>(pow.p, e->jump_digit.p);
@@ -2225,7 +2239,7 @@ int phx_adjoint_device(phx_engine* e, const float* d_gensteps, int32_t num_genst
             }
         }
     if (!e->adj_arr) {
-        int rc = make_texture_f4(e->adj_arr, e->adj_tex, tab, (int)e->nx, (int)e->ny);
+        int rc = make_texture_f4(e->adj_arr, e->adj_tex, tab, (int)e->nx, (int)e->ny, st);
         if (rc) return rc;
     } else {
         PHX_CU(cudaMemcpy2DToArrayAsync(e->adj_arr, 0, 0, tab, e->nx * sizeof(float4), e->nx * sizeof(float4), e->ny,
@@ -2586,7 +2600,8 @@ int phx_set_input_photon(phx_engine* e, const float* photon, int64_t num_photon)
     e->num_input_photon = 0;
     if (num_photon == 0) { e->input_own.release(); return 0; }
     PHX_CU(e->input_own.ensure((size_t)num_photon * 4));
-    PHX_CU(cudaMemcpy(e->input_own.p, photon, (size_t)num_photon * 64, cudaMemcpyHostToDevice));
+    // behind the calls of blocking streams that may still read the previous photons
+    PHX_CU(phx_upload(e->input_own.p, photon, (size_t)num_photon * 64, cudaStreamLegacy));
     e->input_photon = e->input_own.p;
     e->num_input_photon = num_photon;
     return 0;
