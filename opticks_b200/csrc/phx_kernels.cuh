@@ -202,15 +202,14 @@ PHX_D void phx_ray_slabs(const float3& o, const float3& d, PhxSlabs& R)
 // sort key itself.  10M-photon detector event 13.77 -> 13.15 ms against four unpacked slab tests.
 PHX_D void phx_visit_node(const PhxScene& S, int ni, const PhxSlabs& R, float tmin, float tmax, int2* stk, int& sp, unsigned& status)
 {
-    const char* nb = reinterpret_cast<const char*>(S.bvh);
-    const unsigned at = (unsigned)ni << 7;
-    const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + R.nx)));
-    const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + (R.nx ^ 16u))));
-    const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 32u + R.ny)));
-    const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 32u + (R.ny ^ 16u))));
-    const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 64u + R.nz)));
-    const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2*>(nb + (at + 64u + (R.nz ^ 16u))));
-    const int4 ch = __ldg(reinterpret_cast<const int4*>(nb + (at + 96u)));
+    const char* nb = reinterpret_cast<const char*>(S.bvh + ni);
+    const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2*>(nb + R.nx));
+    const ulonglong2 fx = __ldg(reinterpret_cast<const ulonglong2*>(nb + (R.nx ^ 16u)));
+    const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2*>(nb + 32 + R.ny));
+    const ulonglong2 fy = __ldg(reinterpret_cast<const ulonglong2*>(nb + 32 + (R.ny ^ 16u)));
+    const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2*>(nb + 64 + R.nz));
+    const ulonglong2 fz = __ldg(reinterpret_cast<const ulonglong2*>(nb + 64 + (R.nz ^ 16u)));
+    const int4 ch = __ldg(reinterpret_cast<const int4*>(nb + 96));
     const int cha[4] = { ch.x, ch.y, ch.z, ch.w };
     unsigned key[4];
 #pragma unroll
