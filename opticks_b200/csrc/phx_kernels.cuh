@@ -465,27 +465,6 @@ PHX_D void seq_add_nibble(unsigned long long* seqhis, unsigned long long* seqbnd
     }
 }
 
-// The bounce loop of CSGOptiX/CSGOptiX7.cu:432-530 with sctx::point/end seq recording
-// (sysrap/sctx.h:134-185, sysrap/sseq.h:174-184) always on.
-template <int CV>
-PHX_D void phx_bounce_loop(PhxPhoton& p, curandStateXORWOW& rng, const PhxScene& S, const PhxProps& P, const PhxLoopCfg& C,
-                           unsigned long long* seqhis, unsigned long long* seqbnd, unsigned& status)
-{
-    int bounce = 0;
-    seq_add_nibble(seqhis, seqbnd, 0u, p.flag(), p.boundary());
-    while (bounce < C.max_bounce && p.time < C.max_time) {
-        const float tmin = (p.obf & C.eps0_mask) ? C.tmin0 : C.tmin;
-        PhxPRD prd;
-        phx_trace<CV>(S, p.pos, p.mom, tmin, C.tmax, prd, status);
-        if (prd.boundary() == 0xffffu) break;
-        prd.normal = normalize(prd.normal);
-        const int command = propagate(p, rng, prd, P, status);
-        bounce++;
-        seq_add_nibble(seqhis, seqbnd, (unsigned)bounce, p.flag(), p.boundary());
-        if (command == PHX_BREAK) break;
-    }
-}
-
 // genstep of photon idx: the last g with off[g] <= idx (empty gensteps are skipped)
 PHX_D int phx_find_genstep(const long long* off, int G, long long idx)
 {

@@ -164,6 +164,26 @@ PHX_D bool phx_propagate_step(PhxPhoton& p, curandStateXORWOW& rng, const PhxPRD
     return (io.status_command & 0x80000000u) != 0u;
 }
 
+// The bounce loop of CSGOptiX/CSGOptiX7.cu:432-530 with sctx::point/end seq recording
+// (sysrap/sctx.h:134-185, sysrap/sseq.h:174-184) always on.  Through the
+// physics step that the other loop forms call: an inlined copy would round differently.
+template <int CV>
+PHX_D void phx_bounce_loop(PhxPhoton& p, curandStateXORWOW& rng, const PhxScene& S, const PhxProps& P, const PhxLoopCfg& C,
+                           unsigned long long* seqhis, unsigned long long* seqbnd, unsigned& status)
+{
+    int bounce = 0;
+    seq_add_nibble(seqhis, seqbnd, 0u, p.flag(), p.boundary());
+    while (bounce < C.max_bounce && p.time < C.max_time) {
+        const float tmin = (p.obf & C.eps0_mask) ? C.tmin0 : C.tmin;
+        const PhxPRD prd = phx_trace_step<CV>(S, p.pos, p.mom, tmin, C.tmax, status);
+        if (prd.boundary() == 0xffffu) break;
+        const bool ends = phx_propagate_step(p, rng, prd, P, status);
+        bounce++;
+        seq_add_nibble(seqhis, seqbnd, (unsigned)bounce, p.flag(), p.boundary());
+        if (ends) break;
+    }
+}
+
 // The adjoint's physics step out of line, for the loops that hold a path over many bounces: compiled
 // apart from the closest-hit search, its roundings are those of the wavefront's physics kernel (the
 // pathwise terms are differences of nearly equal hits, which any other rounding shows in).

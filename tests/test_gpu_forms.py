@@ -1,0 +1,75 @@
+"""The loop forms (kernel_mode 0: one thread per photon, 1: persistent threads, 2: wavefront) give the same
+photons, seq and hits bit for bit, in geometries of each kind of closest-hit search."""
+import numpy as np
+import pytest
+
+from opticks_b200 import foundry as F
+from opticks_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _detector(n):
+    fd, lib, icdf = scenes.detector()
+    phys = lib.arrays()
+    phys["icdf"] = icdf
+    return fd, phys, scenes.detector_gensteps(1, n, seed=n, lib=lib)
+
+
+def _zoo(n):
+    fd, lib, _, _ = scenes.leaf_zoo_detector(1)
+    return fd, lib.arrays(), scenes.torch_genstep(n, wavelength=440.0, radius=0.0)[None]
+
+
+def filled(world, extra=(), each=20):
+    """bodies throughout the volume, its centre too, so that no ball is free of the hierarchy"""
+    fd = F.Foundry()
+    fd.add_inst(np.eye(4), fd.add_solid("world", [fd.add_prim(world, 0)]))
+    cap = F.op("union", F.zsphere(254.0, 0.0, 190.0), F.cylinder(50.0, -200.0, 0.0))
+    shell = F.op("difference", F.sphere(250.0), F.sphere(150.0))
+    rng = np.random.default_rng(5)
+    for i, b in enumerate([cap, shell, F.sphere(180.0), F.cylinder(90.0, -250.0, 120.0), *extra]):
+        s = fd.add_solid(f"s{i}", [fd.add_prim(b, 1)])
+        for k in range(each):
+            at = rng.uniform(-1800.0, 1800.0, 3) if (i or k) else np.array([30.0, 20.0, 10.0])
+            fd.add_inst(F.look_at_z(at, rng.normal(size=3)), s, sensor_identifier=i, sensor_index=i)
+    return fd
+
+
+def _filled(world, extra=()):
+    def make(n):
+        _, lib, _, _ = scenes.leaf_zoo_detector(1)
+        return filled(world, extra), lib.arrays(), scenes.torch_genstep(n, wavelength=440.0, radius=0.0, pos=(500.0, 300.0, 200.0))[None]
+    return make
+
+
+CONE = F.cone(120.0, -100.0, 60.0, 100.0)
+SCENES = {
+    "detector": _detector,                                                     # plain globals, a ball free of the hierarchy
+    "zoo": _zoo,                                                               # further leaves
+    "sphere world": _filled(F.sphere(4000.0)),                                 # plain global, no ball
+    "cylinder world": _filled(F.cylinder(4000.0, -4000.0, 4000.0)),            # a global leaf without a parameter row
+    "with cones": _filled(F.sphere(4000.0), (CONE,)),                          # the general evaluator in the hierarchy
+}
+
+
+def simulate(E, scene, n, event, **kw):
+    fd, phys, gs = scene(n)
+    eng = E.Engine(fd.arrays(), phys, E.default_config(max_photon=n, **kw))
+    r = eng.simulate(gs, event)
+    r["stats"] = eng.last_call_stats()
+    eng.close()
+    return r
+
+
+def assert_same(a, b):
+    assert a["status"] == 0 and b["status"] == 0
+    for k in ("photon", "seq", "hit"):
+        np.testing.assert_array_equal(a[k].view(np.uint32), b[k].view(np.uint32))
+
+
+@pytest.mark.parametrize("name", SCENES)
+def test_one_thread_per_photon_equals_the_persistent_loop(cuda, name):
+    from opticks_b200 import engine as E
+    a, b = (simulate(E, SCENES[name], 200_000, 3, kernel_mode=m) for m in (0, 1))
+    assert_same(a, b)
