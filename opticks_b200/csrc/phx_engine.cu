@@ -2461,7 +2461,7 @@ static int merge_sorted(phx_engine* e, const uint32_t* in, long long n, uint32_t
     uint32_t* vin = w.val0.p;
     uint32_t* vout = w.val1.p;
     for (int b = 0; b < 8; b++) {
-        if (((b < 4 ? range.bk_max : b < 6 ? 0u : range.id_max) >> (8 * (b < 4 ? b : b - 6))) == 0u) continue;
+        if (!phx_merge_byte_used(range, b)) continue;
         k_radix_hist<<<(unsigned)nt, 256, 0, st>>>(kin, m, 8 * b, w.hist.p, (int)nt);
         if ((rc = merge_scan(w, w.hist.p, 256 * nt, nullptr, st))) return rc;
         k_radix_scatter<<<(unsigned)nt, 256, 0, st>>>(kin, vin, kout, vout, m, 8 * b, w.hist.p, (int)nt);

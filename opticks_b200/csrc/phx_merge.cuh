@@ -97,6 +97,13 @@ __host__ __device__ inline PhxMergeMap phx_merge_map(const PhxMergeRange& r)
     return m;
 }
 
+// does key byte b (0-3 bucket, 4-5 unused, 6-7 identity) hold a bit of any key?
+__host__ __device__ inline bool phx_merge_byte_used(const PhxMergeRange& r, int b)
+{
+    if (b < 4) return (r.bk_max >> (8 * b)) != 0u;
+    return b >= 6 && (r.id_max >> (8 * (b - 6))) != 0u;
+}
+
 #define PHX_MERGE_NONE 0xffffffffffffffffull         // key of a record that is not selected (identities are 16 bits)
 
 template <int LITE>
