@@ -49,13 +49,15 @@ PHX_D bool phx_ball_overlaps(const float4 b, const float3& o, const float3& d, f
 
 // No hit of what the ball (centre, radius) holds can lie on the ray beyond tmin: the line passes it by, or
 // it lies behind the origin.  The margin grows with the origin's distance as the FP32 error of the
-// leaves' own discriminants does, a hundred times wider.  False for any NaN.
+// leaves' own discriminants does, a hundred times wider.  False for any NaN, and where the products of a
+// very long or short direction leave the FP32 range (the leaves' own, smaller products may not).
 PHX_D bool phx_ball_missed(const float4 b, const float3& o, const float3& d, float tmin)
 {
     const float3 oc = make_float3(b.x - o.x, b.y - o.y, b.z - o.z);
     const float dd = dot(d, d), bd = dot(oc, d), cc = dot(oc, oc);
     const float rr = b.w * b.w + 1e-5f * cc;
-    return cc * dd - bd * bd > rr * dd || (bd < 0.f && tmin >= 0.f && cc > rr);
+    const float cd = cc * dd;
+    return (dd > 1e-30f && cd < 3e38f && cd - bd * bd > rr * dd) || (bd < 0.f && tmin >= 0.f && cc > rr);
 }
 
 // IS program of CSGOptiX/CSGOptiX7.cu:896-967 for one (instance, prim) leaf: object-frame
