@@ -98,6 +98,11 @@ struct PhxCsgCtx {
 #define PHX_CV_PLAIN 4
 #define PHX_CV_P(cv) (((cv) & PHX_CV_POLISH) != 0)
 #define PHX_CV_F(cv) (((cv) & PHX_CV_FULL) != 0)
+// The variants whose closest-hit search evaluates the usual prims inline and any other through one call.
+// With the further leaves or the FP64 polish the evaluator's code and registers are there in any
+// case, and a second, inlined form beside it costs more than it saves: 1M photons among bodies of all
+// kinds 10.1 ms with both, 8.6 without the inlined form; the same polished 18.9 and 14.6 ms.
+#define PHX_CV_INLINE(cv) ((cv) == 0 || (cv) == PHX_CV_PLAIN)
 
 // typecodes the base variant evaluates (operators, CSG_ZERO and the five leaves)
 __host__ __device__ inline bool phx_csg_base_typecode(unsigned tc)
@@ -782,14 +787,13 @@ PHX_LEAFFN float4 leaf_eval(const float4* __restrict__ node, const float4* __res
 
 // the sphere, zsphere and cylinder leaves inlined into the caller (closest-hit kernels): no call, so
 // the caller's ray and traversal state need not survive one
-template <bool POLISH>
 PHX_D float4 leaf_fast(const float4* __restrict__ node, const float4* __restrict__ itra, const int ni, const float t_min,
                        const float3& ray_o, const float3& ray_d)
 {
     PHX_LEAF_PROLOGUE
-    if (typecode == PHX_CSG_ZSPHERE) valid = leaf_zsphere<POLISH>(isect, q0, q1, t_min, origin, direction);
-    else if (typecode == PHX_CSG_CYLINDER) valid = leaf_cylinder<POLISH>(isect, q0, q1, t_min, origin, direction);
-    else valid = leaf_sphere<POLISH>(isect, q0, t_min, origin, direction);
+    if (typecode == PHX_CSG_ZSPHERE) valid = leaf_zsphere<false>(isect, q0, q1, t_min, origin, direction);
+    else if (typecode == PHX_CSG_CYLINDER) valid = leaf_cylinder<false>(isect, q0, q1, t_min, origin, direction);
+    else valid = leaf_sphere<false>(isect, q0, t_min, origin, direction);
     PHX_LEAF_EPILOGUE
 }
 
@@ -1021,7 +1025,6 @@ PHX_D bool intersect_tree3(float4& isect, const PhxCsgCtx& g, int root, unsigned
 
 // The same for two leaf_fast leaves, known on the host.  One loop body evaluates a leaf (left, right,
 // then whichever has to be looked at again), so the leaf code is inlined once.
-template <bool POLISH>
 PHX_D float4 intersect_tree3_fast(const float4* __restrict__ node, const float4* __restrict__ itra, int root, unsigned op, float t_min,
                                   const float3& o, const float3& d, unsigned& err)
 {
@@ -1030,7 +1033,7 @@ PHX_D float4 intersect_tree3_fast(const float4* __restrict__ node, const float4*
     float t0 = t_min;
 #pragma unroll 1
     for (int it = 0; it < PHX_TREE3_LOOP_CAP + 1; it++) {
-        const float4 v = leaf_fast<POLISH>(node, itra, root + which, t0, o, d);
+        const float4 v = leaf_fast(node, itra, root + which, t0, o, d);
         if (which == 1) L = v; else R = v;
         if (it == 0) { which = 2; continue; }
         int l_state = phx_classify(L, d, t_min);
@@ -1172,8 +1175,8 @@ PHX_D bool intersect_prim(float4& isect, const PhxCsgCtx& g, int root, float t_m
     return false;
 }
 
-// Any prim, out of line: the closest-hit kernels call it for the leaves whose kind (PHX_KIND_*) is not
-// inlined there.
+// Any prim, out of line: the base variant's closest-hit kernels call it for the leaves whose kind
+// (PHX_KIND_*) is not inlined there.
 struct PhxPrimHit { float4 is; unsigned status; bool valid; };
 template <int CV>
 PHX_COLD PhxPrimHit intersect_prim_any(const float4* __restrict__ node, const float4* __restrict__ itra, const float4* __restrict__ plan,

@@ -62,11 +62,11 @@ PHX_D bool phx_ball_missed(const float4 b, const float3& o, const float3& d, flo
 
 // IS program of CSGOptiX/CSGOptiX7.cu:896-967 for one (instance, prim) leaf: object-frame
 // intersect_prim, keep the closest hit.  `li` indexes the scene's leaves, L is that record.
-// The usual prims (PHX_KIND_LEAF, PHX_KIND_TREE3) are evaluated inline: the kind comes with the leaf,
-// so the chain of dependent node loads that finds it out and the calls per leaf go away.  Identity and
-// lposcost of the hit are looked up once a ray (phx_best_prd), not at every closer hit.  With the plain
-// global leaves below: 10M-photon detector event 13.15 -> 12.27 ms, 2^20 rays through the detector
-// 443 -> 402 us.
+// The usual prims (PHX_KIND_LEAF, PHX_KIND_TREE3) are evaluated inline where PHX_CV_INLINE says so: the
+// kind comes with the leaf, so the chain of dependent node loads that finds it out and the calls per
+// leaf go away.  Identity and lposcost of the hit are looked up once a ray (phx_best_prd), not at every
+// closer hit.  With the plain global leaves below: 10M-photon detector event 13.15 -> 12.27 ms, 2^20 rays
+// through the detector 443 -> 402 us.
 template <int CV>
 PHX_D void phx_test_leaf(const PhxScene& S, const int li, const int4 L, const float3& o, const float3& d, float tmin, PhxBest& B,
                          unsigned& status)
@@ -75,23 +75,27 @@ PHX_D void phx_test_leaf(const PhxScene& S, const int li, const int4 L, const fl
     const float4 m[4] = { __ldg(q + 0), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3) };
     const float3 lo = fx_point(m, o);
     const float3 ld = fx_dir(m, d);
-    const unsigned kind = ((unsigned)L.y & S.kind_mask) >> PHX_LEAF_KIND;
     const int root = (int)((unsigned)L.y & ~S.kind_mask);
     float4 is;
     bool valid;
-    if (kind >= PHX_KIND_TREE3) {
-        is = intersect_tree3_fast<PHX_CV_P(CV)>(S.csg.node, S.csg.itra, root, kind - PHX_KIND_TREE3 + 1u, tmin, lo, ld, status);
-        valid = is.w > 0.f;
-    } else if (kind == PHX_KIND_LEAF) {
-        is = leaf_fast<PHX_CV_P(CV)>(S.csg.node, S.csg.itra, root, tmin, lo, ld);
-        valid = is.w > tmin;
-    } else if constexpr ((CV & PHX_CV_PLAIN) != 0) {
-        return;
+    if constexpr (PHX_CV_INLINE(CV)) {
+        const unsigned kind = ((unsigned)L.y & S.kind_mask) >> PHX_LEAF_KIND;
+        if (kind >= PHX_KIND_TREE3) {
+            is = intersect_tree3_fast(S.csg.node, S.csg.itra, root, kind - PHX_KIND_TREE3 + 1u, tmin, lo, ld, status);
+            valid = is.w > 0.f;
+        } else if (kind == PHX_KIND_LEAF) {
+            is = leaf_fast(S.csg.node, S.csg.itra, root, tmin, lo, ld);
+            valid = is.w > tmin;
+        } else if constexpr ((CV & PHX_CV_PLAIN) != 0) {
+            return;
+        } else {
+            const PhxPrimHit h = intersect_prim_any<CV>(S.csg.node, S.csg.itra, S.csg.plan, root, tmin, lo, ld);
+            is = h.is;
+            valid = h.valid;
+            status |= h.status;
+        }
     } else {
-        const PhxPrimHit h = intersect_prim_any<CV>(S.csg.node, S.csg.itra, S.csg.plan, root, tmin, lo, ld);
-        is = h.is;
-        valid = h.valid;
-        status |= h.status;
+        valid = intersect_prim<CV>(is, S.csg, root, tmin, lo, ld, status);
     }
     // OptiX's interval rule: a report outside [tmin, tmax] is ignored (a convexpolyhedron wholly
     // behind the ray reports valid with t = 0, CSG/csg_intersect_leaf_convexpolyhedron.h:85-101)

@@ -402,9 +402,10 @@ __global__ void __launch_bounds__(128, PHX_WAVE_START_MINB) k_wave_start(WaveArg
 // kernel takes 123 registers and the tail kernel 149: 4 blocks each, and 5 of the tail kernel for large
 // calls (10M photons: tail at 4 blocks 9.76 ms, 5 blocks 9.36, 6 blocks 9.87).  Small calls are the
 // latency of single paths, which the 5-block cap's spills lengthen (50k photons 200 us at 4 blocks, 211
-// at 5; 1M Cerenkov photons 1,167 and 1,150).
-#define PHX_TRACE_MINB(cv) (((cv) & PHX_CV_PLAIN) != 0 ? 4 : 3)
-#define PHX_TAIL_MINB(cv, adj, wide) (!(adj) && ((cv) & PHX_CV_PLAIN) != 0 ? ((wide) ? 5 : 4) : 3)
+// at 5; 1M Cerenkov photons 1,167 and 1,150).  With the FP64 polish 3 blocks spill up to 390 B a thread: 2
+// (polished, among bodies of all kinds: 50k photons 1,423 -> 1,239 us, 1M 14.6 -> 13.9 ms).
+#define PHX_TRACE_MINB(cv) (((cv) & PHX_CV_PLAIN) != 0 ? 4 : PHX_CV_P(cv) ? 2 : 3)
+#define PHX_TAIL_MINB(cv, adj, wide) (!(adj) && ((cv) & PHX_CV_PLAIN) != 0 ? ((wide) ? 5 : 4) : PHX_CV_P(cv) ? 2 : 3)
 #define PHX_TAIL_WIDE (1LL << 19)       // photons of a call from which the 5-block tail kernel runs (with a hierarchy)
 
 // The closest-hit round as a stream of rays (phx_trace_stream): each warp takes the round's live slots 32
