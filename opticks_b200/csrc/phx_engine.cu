@@ -543,12 +543,18 @@ __global__ void __launch_bounds__(128) k_csg_scan(PhxCsgCtx csg, int root, float
     if (st) atomicOr(status, st);
 }
 
+PHX_D void phx_store_prd(float4* out, long long i, const PhxPRD& prd)
+{
+    out[2 * i] = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
+    out[2 * i + 1] = make_float4(prd.lposcost, 0.f, __uint_as_float(prd.ii_id), __uint_as_float(prd.gp_bd));
+}
+
 // idle lanes a warp of k_trace_rays waits for before it takes new rays
 #ifndef PHX_TRACE_REFILL
 #define PHX_TRACE_REFILL 12
 #endif
 // The trace step of simtrace (CSGOptiX/CSGOptiX7.cu:563-603 calls trace(), :112-218): the closest
-// hit of arbitrary rays over the whole geometry, one thread per ray (SoA rays), written as the
+// hit of arbitrary rays over the whole geometry (SoA rays), as a stream of rays, written as the
 // reference's quad2 PRD (sysrap/squad.h:180-245): q0 normal.xyz (world, unnormalised), t;
 // q1 lposcost, 0, iindex<<16|identity, globalPrimIdx<<16|boundary (0xffffffff words: a miss)
 template <int CV>
@@ -556,11 +562,8 @@ __global__ void __launch_bounds__(128, PHX_TRACE_MINB(CV)) k_trace_rays(PhxScene
                                                        float4* prd_out, unsigned* status)
 {
     __shared__ int2 queue[4 * 64];
-    // windows of 32 rays; with fewer rays than lanes, narrower ones over all warps (less divergence)
-    const long long warps = 4ll * gridDim.x;
-    const long long width = min(32ll, (n + warps - 1) / warps);
-    long long at = width * ((long long)blockIdx.x * 4 + (threadIdx.x >> 5));      // the warp's next window
-    const long long stride = width * warps;
+    long long at = 32ll * ((long long)blockIdx.x * 4 + (threadIdx.x >> 5));      // the warp's next window of 32 rays
+    const long long stride = 128ll * gridDim.x;
     unsigned st = 0;
     phx_trace_stream<CV>(
         S, t_max, PHX_TRACE_REFILL, queue + 64 * (threadIdx.x >> 5), st,
@@ -571,17 +574,32 @@ __global__ void __launch_bounds__(128, PHX_TRACE_MINB(CV)) k_trace_rays(PhxScene
         },
         [&](long long base, unsigned lane, unsigned& i) {
             i = (unsigned)(base + lane);
-            return (long long)lane < width && base + lane < n;
+            return base + lane < n;
         },
         [&](unsigned i, float3& o, float3& d, float& tmin) {
             o = make_float3(__ldg(rays + i), __ldg(rays + n + i), __ldg(rays + 2 * n + i));
             d = make_float3(__ldg(rays + 3 * n + i), __ldg(rays + 4 * n + i), __ldg(rays + 5 * n + i));
             tmin = t_min;
         },
-        [&](unsigned i, const PhxPRD& prd) {
-            prd_out[2 * (size_t)i] = make_float4(prd.normal.x, prd.normal.y, prd.normal.z, prd.distance);
-            prd_out[2 * (size_t)i + 1] = make_float4(prd.lposcost, 0.f, __uint_as_float(prd.ii_id), __uint_as_float(prd.gp_bd));
-        });
+        [&](unsigned i, const PhxPRD& prd) { phx_store_prd(prd_out, i, prd); });
+    if (st) atomicOr(status, st);
+}
+
+// The same, one thread per ray, `width` rays a warp.  Where every ray has a lane from the start there is
+// nothing to refill, and the stream's two stores, queue and second load of a ray lengthen the call.
+template <int CV>
+__global__ void __launch_bounds__(128, (CV & PHX_CV_PLAIN) != 0 ? 4 : 3) k_trace_each(PhxScene S, const float* rays, long long n, int width, float t_min,
+                                                                        float t_max, float4* prd_out, unsigned* status)
+{
+    const int lane = threadIdx.x & 31;
+    const long long i = (long long)width * ((long long)blockIdx.x * 4 + (threadIdx.x >> 5)) + lane;
+    if (lane >= width || i >= n) return;
+    const float3 o = make_float3(__ldg(rays + i), __ldg(rays + n + i), __ldg(rays + 2 * n + i));
+    const float3 d = make_float3(__ldg(rays + 3 * n + i), __ldg(rays + 4 * n + i), __ldg(rays + 5 * n + i));
+    unsigned st = 0;
+    PhxPRD prd;
+    phx_trace<CV>(S, o, d, t_min, t_max, prd, st);
+    phx_store_prd(prd_out, i, prd);
     if (st) atomicOr(status, st);
 }
 
@@ -1731,15 +1749,26 @@ static int launch_scan_t(int device, const PhxCsgCtx& csg, int root, float t_min
     return 0;
 }
 
+// Queries of at most this many rays take one thread per ray: 1,000 rays through the detector 24.7 us
+// against 28.1 as a stream, 100k 29.2 / 33.6, 200k 31.1 / 36.5, 500k 41.8 / 44.0; among bodies throughout the
+// volume 130k 78.5 / 79.9, 300k 143.1 / 135.7, with cones 20k 48.4 / 63.9, 300k 208.7 / 244.9.
+#define PHX_TRACE_EACH (1LL << 18)
 template <int CV>
 static int launch_trace_t(int device, const PhxScene& S, const float* d_rays, long long n, float t_min, float t_max, float4* out, unsigned* status,
                            cudaStream_t st)
 {
-    static int grid[128] = {};
+    static int grid[128] = {}, grid_each[128] = {};
     if (device < 0 || device >= 128) return phx_fail(-1, "device ordinal %d out of range", device);
-    int rc = wave_grid(k_trace_rays<CV>, device, grid);
-    if (rc) return rc;
-    k_trace_rays<CV><<<(unsigned)std::min<long long>(grid[device], (n + 3) / 4), 128, 0, st>>>(S, d_rays, n, t_min, t_max, out, status);
+    int rc;
+    if (n <= PHX_TRACE_EACH) {
+        if ((rc = wave_grid(k_trace_each<CV>, device, grid_each))) return rc;
+        const long long warps = 4LL * grid_each[device];            // few rays: narrower warps over all of them
+        const int width = (int)std::min<long long>(32, (n + warps - 1) / warps);
+        k_trace_each<CV><<<(unsigned)((n + 4 * width - 1) / (4 * width)), 128, 0, st>>>(S, d_rays, n, width, t_min, t_max, out, status);
+        return 0;
+    }
+    if ((rc = wave_grid(k_trace_rays<CV>, device, grid))) return rc;
+    k_trace_rays<CV><<<(unsigned)std::min<long long>(grid[device], (n + 127) / 128), 128, 0, st>>>(S, d_rays, n, t_min, t_max, out, status);
     return 0;
 }
 

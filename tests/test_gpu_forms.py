@@ -73,3 +73,22 @@ def test_one_thread_per_photon_equals_the_persistent_loop(cuda, name):
     from opticks_b200 import engine as E
     a, b = (simulate(E, SCENES[name], 200_000, 3, kernel_mode=m) for m in (0, 1))
     assert_same(a, b)
+
+
+# ---------------------------------------------------------------- closest hits
+@pytest.mark.parametrize("polish", [0, 1])
+@pytest.mark.parametrize("name", ["detector", "zoo", "sphere world", "with cones"])
+def test_trace_in_pieces(cuda, name, polish):
+    """a query of one ray more than the one-thread-per-ray rule takes (a stream of rays) against its pieces"""
+    from opticks_b200 import engine as E
+    fd, phys, _ = SCENES[name](1)
+    eng = E.Engine(fd.arrays(), phys, E.default_config(max_photon=64, root_polish=polish))
+    n = (1 << 18) + 1
+    rays = scenes.scan_rays(n, seed=5, half=11000.0 if name == "detector" else 1400.0)
+    whole, st = eng.trace(rays, 0.05)
+    assert st == 0
+    cuts = [0, 1, 1000, 1 << 17, n]
+    for a, b in zip(cuts, cuts[1:]):
+        piece, _ = eng.trace(np.ascontiguousarray(rays[:, a:b]), 0.05)
+        np.testing.assert_array_equal(piece.view(np.uint32), whole[a:b].view(np.uint32))
+    eng.close()

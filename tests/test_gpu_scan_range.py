@@ -86,14 +86,15 @@ def test_intervals_that_open_behind_the_origin(cuda):
         assert np.mean(np.abs(g[both, 3] - ref[both, 3]) <= 0.1) >= 0.99
 
 
-def test_trace_of_rays_that_are_no_numbers(cuda):
-    """in the ray stream a NaN ray neither holds up nor changes the others"""
+@pytest.mark.parametrize("n", [30_001, 300_001])              # one thread per ray; the stream of rays
+def test_trace_of_rays_that_are_no_numbers(cuda, n):
+    """a NaN ray neither holds up nor changes the others"""
     from opticks_b200 import engine as E
     fd, lib, icdf = scenes.detector()
     phys = lib.arrays()
     phys["icdf"] = icdf
     eng = E.Engine(fd.arrays(), phys, E.default_config(max_photon=64))
-    rays = scenes.scan_rays(30_001, seed=2, half=11000.0)
+    rays = scenes.scan_rays(n, seed=2, half=11000.0)
     base = rays.copy()
     rays[1, 4::9] = np.nan
     rays[3:, 7::31] = np.nan
