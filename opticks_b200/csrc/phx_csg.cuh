@@ -151,6 +151,13 @@ PHX_D float3 fx_unit(const float3& v) { return fx_scale(v, 1.0f / sqrtf(fx_dot(v
 PHX_D float3 fx_unit_mix(const float3& v) { return fx_scale(v, 1.0f / sqrtf(fx_mix(v.x, v.x, v.y, v.y, v.z, v.z))); }
 // discriminant b b - d c
 PHX_D float fx_disc(float d, float b, float c) { return __fmaf_rn(b, b, -__fmul_rn(d, c)); }
+// the same of the FP64 polish, which is inlined in as many kernels
+PHX_D double fx_dot(double ax, double ay, double az, double bx, double by, double bz)
+{
+    return __fma_rn(az, bz, __fma_rn(ay, by, __dmul_rn(ax, bx)));
+}
+PHX_D double fx_dot2(double ax, double ay, double bx, double by) { return __fma_rn(ay, by, __dmul_rn(ax, bx)); }
+PHX_D double fx_disc(double d, double b, double c) { return __fma_rn(b, b, -__dmul_rn(d, c)); }
 
 // ---------------------------------------------------------------- quadratic roots
 // Solve d t^2 + 2 b t + c = 0 choosing the form of each root that avoids cancellation.
@@ -180,7 +187,7 @@ PHX_D void robust_roots_disq(const float t_min, float& t1, float& t2, float& dis
 // hit/miss topology matches the FP32 path unless the FP32 discriminant itself was wrong.
 PHX_D void polish_roots(float& t1, float& t2, double d, double b, double c)
 {
-    double disc = b * b - d * c;
+    double disc = fx_disc(d, b, c);
     if (disc <= 0.0) return;
     double sd = sqrt(disc);
     double q = b > 0.0 ? -(b + sd) : -(b - sd);
@@ -204,9 +211,9 @@ PHX_D bool leaf_sphere(float4& isect, const float4& q0, float t_min, const float
     robust_roots(root1, root2, disc, sdisc, d, b, c);
     if (POLISH && sdisc > 0.f) {
         double ox = (double)o.x - center.x, oy = (double)o.y - center.y, oz = (double)o.z - center.z;
-        double bb = ox * D.x + oy * D.y + oz * D.z;
-        double cc = ox * ox + oy * oy + oz * oz - (double)radius * radius;
-        double dd = (double)D.x * D.x + (double)D.y * D.y + (double)D.z * D.z;
+        double bb = fx_dot(ox, oy, oz, D.x, D.y, D.z);
+        double cc = __fma_rn(-(double)radius, radius, fx_dot(ox, oy, oz, ox, oy, oz));
+        double dd = fx_dot((double)D.x, D.y, D.z, D.x, D.y, D.z);
         polish_roots(root1, root2, dd, bb, cc);
     }
     float t_cand = sdisc > 0.f ? (root1 > t_min ? root1 : root2) : t_min;
@@ -238,9 +245,9 @@ PHX_D bool leaf_zsphere(float4& isect, const float4& q0, const float4& q1, float
     robust_roots(t1sph, t2sph, disc, sdisc, d, b, c);
     if (POLISH && sdisc > 0.f) {
         double ox = (double)o.x - center.x, oy = (double)o.y - center.y, oz = (double)o.z - center.z;
-        double bb = ox * D.x + oy * D.y + oz * D.z;
-        double cc = ox * ox + oy * oy + oz * oz - (double)radius * radius;
-        double dd = (double)D.x * D.x + (double)D.y * D.y + (double)D.z * D.z;
+        double bb = fx_dot(ox, oy, oz, D.x, D.y, D.z);
+        double cc = __fma_rn(-(double)radius, radius, fx_dot(ox, oy, oz, ox, oy, oz));
+        double dd = fx_dot((double)D.x, D.y, D.z, D.x, D.y, D.z);
         polish_roots(t1sph, t2sph, dd, bb, cc);
     }
     float z1sph = __fmaf_rn(t1sph, dir.z, o.z);
@@ -291,9 +298,9 @@ PHX_D bool leaf_cylinder(float4& isect, const float4& q0, const float4& q1, floa
     float t_near, t_far, disc, sdisc;
     robust_roots_disq(t_min, t_near, t_far, disc, sdisc, a, b, c);
     if (POLISH && sdisc > 0.f) {
-        double aa = (double)vx * vx + (double)vy * vy;
-        double bb = (double)ox * vx + (double)oy * vy;
-        double cc = (double)ox * ox + (double)oy * oy - (double)r * r;
+        double aa = fx_dot2((double)vx, (double)vy, (double)vx, (double)vy);
+        double bb = fx_dot2((double)ox, (double)oy, (double)vx, (double)vy);
+        double cc = __fma_rn(-(double)r, (double)r, fx_dot2((double)ox, (double)oy, (double)ox, (double)oy));
         polish_roots(t_near, t_far, aa, bb, cc);
     }
     float z_near = __fmaf_rn(t_near, vz, oz);

@@ -92,3 +92,57 @@ def test_trace_in_pieces(cuda, name, polish):
         piece, _ = eng.trace(np.ascontiguousarray(rays[:, a:b]), 0.05)
         np.testing.assert_array_equal(piece.view(np.uint32), whole[a:b].view(np.uint32))
     eng.close()
+
+
+# ---------------------------------------------------------------- root polish
+@pytest.mark.parametrize("name,n", [("detector", 16_383), ("detector", 16_384), ("detector", 524_288), ("zoo", 50_000),
+                                    ("sphere world", 300_000), ("cylinder world", 50_000), ("with cones", 300_000)])
+def test_polished_forms_agree(cuda, name, n):
+    """root_polish: the starting kernel's own sphere, the tail kernel, the rounds and the one-kernel loops"""
+    from opticks_b200 import engine as E
+    ref = simulate(E, SCENES[name], n, 3, kernel_mode=1, root_polish=1)
+    for mode in (0, 2):
+        assert_same(simulate(E, SCENES[name], n, 3, kernel_mode=mode, root_polish=1), ref)
+
+
+# ---------------------------------------------------------------- fixed rounds
+@pytest.mark.parametrize("name", ["sphere world", "cylinder world", "with cones"])
+@pytest.mark.parametrize("rounds", [2, 3])
+@pytest.mark.parametrize("polish", [0, 1])
+def test_fixed_rounds_equal_the_persistent_loop(cuda, name, rounds, polish):
+    """more photons than the small-call rule takes, and no ball or a global leaf without a parameter row: rounds of
+    a closest-hit and a physics kernel, then the tail kernel"""
+    from opticks_b200 import engine as E
+    n = 262_145
+    ref = simulate(E, SCENES[name], n, 2, kernel_mode=1, root_polish=polish)
+    got = simulate(E, SCENES[name], n, 2, kernel_mode=2, root_polish=polish, wave_rounds=rounds)
+    assert got["stats"]["wave_rounds"] == rounds          # the schedule this test is about
+    assert_same(got, ref)
+
+
+@pytest.mark.parametrize("name", ["sphere world", "with cones"])
+def test_captured_fixed_rounds(cuda, name):
+    """the same in a batched call, captured as a graph and replayed"""
+    from opticks_b200 import engine as E
+    torch = cuda
+    fd, phys, _ = SCENES[name](1)
+    counts = [100_000, 1, 70_000, 110_000]
+    gs = np.concatenate([scenes.torch_genstep(c, wavelength=440.0, radius=0.0, pos=(500.0, 300.0, 200.0))[None] for c in counts])
+    N = sum(counts)
+    g, ev = torch.from_numpy(gs).cuda(), torch.arange(3, 3 + len(counts), dtype=torch.int32, device="cuda")
+    outs = []
+    for mode, calls in ((1, 1), (2, 3)):
+        eng = E.Engine(fd.arrays(), phys, E.default_config(max_photon=max(counts), kernel_mode=mode, wave_rounds=2, use_graph=1))
+        ph = torch.empty((N, 4, 4), dtype=torch.float32, device="cuda")
+        sq = torch.empty((N, 2, 2), dtype=torch.int64, device="cuda")
+        for _ in range(calls):
+            ph.fill_(0.0)
+            sq.fill_(0)
+            _, st = eng.simulate_batched_device(g, ev, N, photon=ph, seq=sq, stream=torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            assert st == 0
+        stats = eng.last_call_stats()
+        eng.close()
+        outs.append((ph.clone(), sq.clone()))
+    assert stats["graph"] == 1
+    assert torch.equal(outs[0][0].view(torch.int32), outs[1][0].view(torch.int32)) and torch.equal(outs[0][1], outs[1][1])
