@@ -2454,9 +2454,17 @@ extern "C" int phx_simulate_device_noalloc(phx_engine* e, const float* d_genstep
 }
 
 // ------------------------------------------------------------------ hit merging
-// exclusive scan of n u32 in place; the total goes to *d_total when given
+// exclusive scan of n u32 in place; the total goes to *d_total when given.  Up to
+// PHX_MERGE_SCAN_ONE words are scanned by one block, 1024 a turn, in place of three launches.
+#define PHX_MERGE_SCAN_ONE 8192
 static int merge_scan(PhxMergeWs& w, uint32_t* x, long long n, long long* d_total, cudaStream_t st)
 {
+    if (n <= PHX_MERGE_SCAN_ONE) {
+        PHX_CU(w.total.ensure(2));
+        k_block_scan<<<1, 1024, 0, st>>>(x, (int)n, d_total ? d_total : w.total.p + 1);
+        PHX_CU(cudaGetLastError());
+        return 0;
+    }
     const long long nt = (n + PHX_MERGE_SCAN_TILE - 1) / PHX_MERGE_SCAN_TILE;
     PHX_CU(w.tsum.ensure((size_t)std::max(1LL, nt)));
     PHX_CU(w.total.ensure(2));
@@ -2476,47 +2484,64 @@ static int merge_read(phx_engine* e, const void* d, size_t bytes, void* h, cudaS
     return 0;
 }
 
-// ordered positions of the records `mask` selects, in w.sel (null with every record selected)
+// ordered positions of the records `mask` selects, in w.sel (null with every record selected); with `key` (the
+// keys of all n records, PHX_MERGE_NONE where not selected) also their keys, in sel_key
 template <int LITE>
-static int merge_select(PhxMergeWs& w, const uint32_t* in, long long n, uint32_t mask, const uint32_t** sel, cudaStream_t st)
+static int merge_select(PhxMergeWs& w, const uint32_t* in, const unsigned long long* key, long long n, uint32_t mask, long long room,
+                        unsigned long long* sel_key, const uint32_t** sel, cudaStream_t st)
 {
     *sel = nullptr;
     if (mask == 0xffffffffu) return 0;
     const long long nt = (n + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE;
     PHX_CU(w.total.ensure(2));
     PHX_CU(w.tcount.ensure((size_t)nt));
-    PHX_CU(w.sel.ensure((size_t)n));
-    k_merge_sel_count<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p);
+    PHX_CU(w.sel.ensure((size_t)room));
+    k_merge_sel_count<LITE><<<(unsigned)nt, 256, 0, st>>>(in, key, n, mask, w.tcount.p);
     k_block_scan<<<1, 1024, 0, st>>>(w.tcount.p, (int)nt, w.total.p);
-    k_merge_sel_write<LITE><<<(unsigned)nt, 256, 0, st>>>(in, n, mask, w.tcount.p, w.sel.p);
+    k_merge_sel_write<LITE><<<(unsigned)nt, 256, 0, st>>>(in, key, n, mask, w.tcount.p, w.sel.p, sel_key);
     PHX_CU(cudaGetLastError());
     *sel = w.sel.p;
     return 0;
 }
 
-// the sort form of merge_impl (phx_merge.cuh) for keys whose range no table holds
+// scratch of the sort form for m selected records, beside the keys
+static cudaError_t merge_sort_room(PhxMergeWs& w, long long m)
+{
+    const size_t M = (size_t)m;
+    cudaError_t e = w.key1.ensure(M);
+    if (e == cudaSuccess) e = w.val0.ensure(M);
+    if (e == cudaSuccess) e = w.val1.ensure(M);
+    if (e == cudaSuccess) e = w.sel.ensure(M);
+    if (e == cudaSuccess) e = w.head.ensure(M);
+    if (e == cudaSuccess) e = w.hist.ensure(256 * ((M + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE));
+    return e;
+}
+
+// The sort form of merge_impl (phx_merge.cuh) for keys whose range no table holds.  With `tried`, the
+// table form's first step has left the keys in w.key0, and they are taken over.
 template <int LITE>
-static int merge_sorted(phx_engine* e, const uint32_t* in, long long n, uint32_t mask, float tw, const PhxMergeRange& range, uint32_t* out,
-                        long long cap, long long* num_out, cudaStream_t st)
+static int merge_sorted(phx_engine* e, const uint32_t* in, long long n, uint32_t mask, float tw, const PhxMergeRange& range, bool tried,
+                        uint32_t* out, long long cap, long long* num_out, cudaStream_t st)
 {
     PhxMergeWs& w = e->merge;
-    const uint32_t* sel = nullptr;
-    int rc = merge_select<LITE>(w, in, n, mask, &sel, st);
-    if (rc) return rc;
     const long long m = (long long)range.count;
     const unsigned grid = (unsigned)std::min<long long>((m + 255) / 256, 148LL * 16);
     PHX_CU(w.total.ensure(2));
-    PHX_CU(w.key0.ensure((size_t)m)); PHX_CU(w.key1.ensure((size_t)m));
-    PHX_CU(w.val0.ensure((size_t)m)); PHX_CU(w.val1.ensure((size_t)m));
-    k_merge_keys<LITE><<<grid, 256, 0, st>>>(in, sel, m, tw, w.key0.p, w.val0.p);
-    PHX_CU(cudaGetLastError());
+    PHX_CU(w.key0.ensure((size_t)m));
+    PHX_CU(merge_sort_room(w, m));
+    const uint32_t* vin = nullptr;               // input positions of the keys (null: 0, 1, ...)
+    int rc = merge_select<LITE>(w, in, tried ? w.key0.p : nullptr, n, mask, m, tried ? w.key1.p : nullptr, &vin, st);
+    if (rc) return rc;
+    unsigned long long* kin = tried && vin ? w.key1.p : w.key0.p;
+    unsigned long long* kout = kin == w.key0.p ? w.key1.p : w.key0.p;
+    uint32_t* vout = w.val0.p;
+    uint32_t* vnext = w.val1.p;
+    if (!tried) {
+        k_merge_keys<LITE><<<grid, 256, 0, st>>>(in, vin, m, tw, kin);
+        PHX_CU(cudaGetLastError());
+    }
     // stable LSD radix passes over the key bytes up to the largest bucket and identity
     const long long nt = (m + PHX_MERGE_TILE - 1) / PHX_MERGE_TILE;
-    PHX_CU(w.hist.ensure((size_t)(256 * nt)));
-    unsigned long long* kin = w.key0.p;
-    unsigned long long* kout = w.key1.p;
-    uint32_t* vin = w.val0.p;
-    uint32_t* vout = w.val1.p;
     for (int b = 0; b < 8; b++) {
         if (!phx_merge_byte_used(range, b)) continue;
         k_radix_hist<<<(unsigned)nt, 256, 0, st>>>(kin, m, 8 * b, w.hist.p, (int)nt);
@@ -2524,26 +2549,45 @@ static int merge_sorted(phx_engine* e, const uint32_t* in, long long n, uint32_t
         k_radix_scatter<<<(unsigned)nt, 256, 0, st>>>(kin, vin, kout, vout, m, 8 * b, w.hist.p, (int)nt);
         PHX_CU(cudaGetLastError());
         std::swap(kin, kout);
-        std::swap(vin, vout);
+        vin = vout;
+        std::swap(vout, vnext);
     }
     // groups
-    PHX_CU(w.head.ensure((size_t)m));
     k_merge_heads<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(kin, m, w.head.p);
     if ((rc = merge_scan(w, w.head.p, m, w.total.p, st))) return rc;
     long long ng = 0;
     if ((rc = merge_read(e, w.total.p, sizeof(long long), &ng, st))) return rc;
     *num_out = ng;
     if (ng > cap) return phx_fail(-3, "phx_merge_hits: %lld merged records, out_capacity %lld", ng, cap);
-    PHX_CU(w.amin.ensure((size_t)ng)); PHX_CU(w.pmin.ensure((size_t)ng));
-    PHX_CU(w.gor.ensure((size_t)ng)); PHX_CU(w.gsum.ensure((size_t)ng));
-    PHX_CU(cudaMemsetAsync(w.amin.p, 0xff, sizeof(unsigned long long) * ng, st));
-    PHX_CU(cudaMemsetAsync(w.pmin.p, 0xff, sizeof(uint32_t) * ng, st));
-    PHX_CU(cudaMemsetAsync(w.gor.p, 0, sizeof(uint32_t) * ng, st));
-    PHX_CU(cudaMemsetAsync(w.gsum.p, 0, sizeof(uint32_t) * ng, st));
-    k_merge_reduce<LITE><<<grid, 256, 0, st>>>(in, sel, kin, vin, w.head.p, m, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
-    k_merge_write<LITE><<<(unsigned)((ng + 255) / 256), 256, 0, st>>>(in, sel, ng, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p, out);
+    PHX_CU(w.amin.ensure((size_t)ng)); PHX_CU(w.gor.ensure((size_t)ng)); PHX_CU(w.gsum.ensure((size_t)ng));
+    if (LITE) PHX_CU(w.pmin.ensure((size_t)ng));
+    k_merge_clear<LITE><<<(unsigned)((ng + 255) / 256), 256, 0, st>>>(ng, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
+    k_merge_reduce<LITE><<<grid, 256, 0, st>>>(in, kin, vin, w.head.p, m, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
+    k_merge_write<LITE><<<(unsigned)((ng + 255) / 256), 256, 0, st>>>(in, ng, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p, out);
     PHX_CU(cudaGetLastError());
     return 0;
+}
+
+static void merge_table_release(PhxMergeWs& w)
+{
+    cudaGetLastError();              // (the failed allocation that led here)
+    w.cell.release(); w.cell_off.release(); w.cell_blk.release();
+    w.key0.release(); w.amin.release(); w.gor.release(); w.gsum.release(); w.pmin.release();
+}
+
+// scratch of the table form for n records
+static cudaError_t merge_table_room(PhxMergeWs& w, long long n, long long ncw, bool lite)
+{
+    const size_t N = (size_t)n;
+    cudaError_t e = w.cell.ensure((size_t)ncw);
+    if (e == cudaSuccess) e = w.cell_off.ensure((size_t)ncw);
+    if (e == cudaSuccess) e = w.cell_blk.ensure((size_t)ncw / 1024);
+    if (e == cudaSuccess) e = w.key0.ensure(N);
+    if (e == cudaSuccess) e = w.amin.ensure(N);
+    if (e == cudaSuccess) e = w.gor.ensure(N);
+    if (e == cudaSuccess) e = w.gsum.ensure(N);
+    if (e == cudaSuccess && lite) e = w.pmin.ensure(N);
+    return e;
 }
 
 template <int LITE>
@@ -2557,7 +2601,7 @@ static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t m
     if (tw == 0.f) {                 // selection only, input order
         const int W = PhxRec<LITE>::W;
         const uint32_t* sel = nullptr;
-        if ((rc = merge_select<LITE>(w, in, n, mask, &sel, st))) return rc;
+        if ((rc = merge_select<LITE>(w, in, nullptr, n, mask, n, nullptr, &sel, st))) return rc;
         long long m = n;
         if (sel && (rc = merge_read(e, w.total.p, sizeof(long long), &m, st))) return rc;
         if (m == 0) return 0;
@@ -2567,29 +2611,40 @@ static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t m
         PHX_CU(cudaGetLastError());
         return 0;
     }
-    // table form, decided on the device: every kernel leaves at once when the range has more cells
-    // than the table, and the sort form takes over after the one host read
+    // Table form, decided on the device: every kernel leaves at once when the range has more cells
+    // than the table, and the sort form takes over after the one host read.  Its scratch goes with the
+    // input records, the sort form's with the selected ones: where memory is short the sort form runs
+    // alone, after the range.
     const unsigned long long most = phx_merge_cells(n);
     const long long ncw = (long long)(most / 32ull), nblk = ncw / 1024;
-    PHX_CU(w.range.ensure(1));
-    PHX_CU(w.cell.ensure((size_t)ncw)); PHX_CU(w.cell_off.ensure((size_t)ncw)); PHX_CU(w.cell_blk.ensure((size_t)nblk));
-    PHX_CU(w.key0.ensure((size_t)n)); PHX_CU(w.amin.ensure((size_t)n));
-    PHX_CU(w.gor.ensure((size_t)n)); PHX_CU(w.gsum.ensure((size_t)n));
-    if (LITE) PHX_CU(w.pmin.ensure((size_t)n));
-    PHX_CU(cudaMemsetAsync(w.range.p, 0, sizeof(PhxMergeRange), st));
     const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 8);
-    k_merge_range<LITE><<<std::max(grid, 148u), 256, 0, st>>>(in, n, mask, tw, w.key0.p, w.range.p, w.cell.p, ncw, w.amin.p, w.pmin.p, w.gor.p,
-                                                              w.gsum.p);
-    k_merge_present<<<grid, 256, 0, st>>>(w.key0.p, n, w.range.p, most, w.cell.p);
+    PhxMergeRange range;
+    PHX_CU(w.range.ensure(1));
+    PHX_CU(cudaMemsetAsync(w.range.p, 0, sizeof(PhxMergeRange), st));
+    const cudaError_t room = merge_table_room(w, n, ncw, LITE != 0);
+    if (room == cudaErrorMemoryAllocation) {
+        merge_table_release(w);
+        k_merge_range<LITE><<<grid, 256, 0, st>>>(in, n, mask, tw, nullptr, w.range.p, nullptr, 0);
+        PHX_CU(cudaGetLastError());
+        if ((rc = merge_read(e, w.range.p, sizeof(range), &range, st))) return rc;
+        if (range.count == 0ull) return 0;
+        return merge_sorted<LITE>(e, in, n, mask, tw, range, false, out, cap, num_out, st);
+    }
+    PHX_CU(room);
+    k_merge_range<LITE><<<std::max(grid, 148u), 256, 0, st>>>(in, n, mask, tw, w.key0.p, w.range.p, w.cell.p, ncw);
+    k_merge_present<LITE><<<grid, 256, 0, st>>>(w.key0.p, n, w.range.p, most, w.cell.p, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
     k_merge_rank<<<(unsigned)nblk, 256, 0, st>>>(w.cell.p, w.range.p, most, w.cell_off.p, w.cell_blk.p);
     k_block_scan<<<1, 1024, 0, st>>>(w.cell_blk.p, (int)nblk, &w.range.p->groups);
     k_merge_fold<LITE><<<grid, 256, 0, st>>>(in, w.key0.p, n, w.range.p, most, w.cell.p, w.cell_off.p, w.cell_blk.p, w.amin.p, w.pmin.p,
                                              w.gor.p, w.gsum.p);
     k_merge_groups<LITE><<<grid, 256, 0, st>>>(in, w.range.p, most, cap, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p, out);
     PHX_CU(cudaGetLastError());
-    PhxMergeRange range;
     if ((rc = merge_read(e, w.range.p, sizeof(range), &range, st))) return rc;
-    if (phx_merge_map(range).cells > most) return merge_sorted<LITE>(e, in, n, mask, tw, range, out, cap, num_out, st);
+    if (phx_merge_map(range).cells > most) {
+        const bool fits = merge_sort_room(w, (long long)range.count) != cudaErrorMemoryAllocation;
+        if (!fits) merge_table_release(w);
+        return merge_sorted<LITE>(e, in, n, mask, tw, range, fits, out, cap, num_out, st);
+    }
     *num_out = range.groups;
     if (range.groups > cap) return phx_fail(-3, "phx_merge_hits: %lld merged records, out_capacity %lld", range.groups, cap);
     return 0;

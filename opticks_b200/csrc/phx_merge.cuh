@@ -24,15 +24,22 @@
 // in one go without a host read (the table's size comes from n, the range stays on the device).  1M
 // sphoton records with a fifth selected, 1 ns windows: 79 us a call, against 247 us through the sort
 // (35 launches and three host reads); what is left is six launches and one read at 4-20 us apiece.
-// Ranges whose cells outnumber the table (phx_merge_cells) are left to a stable sort of the keys:
-//   1. ordered selection (ballot + tile offsets)           -> sel[m] input positions
-//   2. keys (u64); passes only over the key bytes in use
+// Ranges whose cells outnumber the table (phx_merge_cells) are left to a stable sort of the keys.  They are
+// ordinary: with 17,612 sensors the 2^24 cells of a small event are 952 buckets, so one microsecond-late
+// selected record at 1 ns is enough.  The failed attempt (a read of the records and five launches that leave
+// at once) is paid back by its keys: 4M records, a fifth selected, 433 us before there was a table, 500 with
+// the sort started over, 396 with the keys taken over; 100,000 all selected 212, 236, 225; 1,000 162, 192, 152.
+//   1. ordered selection from the keys (ballot + tile offsets) -> input positions and keys
+//   2. passes only over the key bytes in use
 //   3. stable LSD radix sort, 8-bit digits: per-tile digit histograms (digit-major), one scan,
 //      a scatter ranking equal digits by __match_any_sync so every pass is stable
 //   4. group heads + scan -> group index; warp-segmented reductions (__reduce_*_sync over the
 //      lanes of one group) with one atomic per (warp, group): min (time, position), min position,
 //      OR flagmask, sum hitcount
 //   5. one thread per group writes the representative record with the reduced fields
+// Scratch: the table form takes 24 B an input record (28 for sphotonlite) and the table, the sort form 25 B a
+// selected record besides.  Where either has no room in device memory the range alone is found and the
+// sort form starts from the records, at 33 B a selected one and 16 to 20 a group.
 // Each form picks the record the left fold of reduce_op picks.  Included by phx_engine.cu after
 // DevBuf and PHX_CU.
 #pragma once
@@ -66,8 +73,9 @@ __device__ __forceinline__ uint32_t phx_time_unorder(uint32_t o)
 }
 
 // ---------------------------------------------------------------- table form
-// Bits of the cell table for n records: 32 per record, and never fewer than 2^24 (2 MB).  The table
-// is cleared and scanned on each call at 4 B per record, an eighth of the least the records cost.
+// Bits of the cell table for n records: 32 per record (4 B), and never fewer than 2^24 (2 MB).  The
+// whole table is cleared on each call, and the range's part of it read and its offsets written (8 B a
+// word): against a 16 B record at most three quarters of its bytes, below 524,288 records 2 MB whatever n.
 __host__ __device__ inline unsigned long long phx_merge_cells(long long n)
 {
     const unsigned long long c = 32ull * (unsigned long long)n;
@@ -114,11 +122,19 @@ __device__ __forceinline__ unsigned long long phx_merge_key(const uint32_t* r, f
     return ((unsigned long long)id << 48) | (unsigned long long)bucket;
 }
 
-// 1. keys and their ranges; also clears the cell table and the n group slots
+template <int LITE>
+__device__ __forceinline__ void phx_merge_clear(long long g, unsigned long long* amin, uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
+{
+    amin[g] = 0xffffffffffffffffull;
+    if (LITE) pmin[g] = 0xffffffffu;
+    gor[g] = 0u;
+    gsum[g] = 0u;
+}
+
+// 1. keys and their ranges; also clears the cell table (key null: the range alone)
 template <int LITE>
 __global__ void __launch_bounds__(256) k_merge_range(const uint32_t* in, long long n, uint32_t mask, float tw, unsigned long long* key,
-                                                     PhxMergeRange* range, uint32_t* cell, long long ncellw, unsigned long long* amin,
-                                                     uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
+                                                     PhxMergeRange* range, uint32_t* cell, long long ncellw)
 {
     __shared__ uint32_t s_id, s_idc, s_bk, s_bkc, s_cnt;
     if (threadIdx.x == 0) s_id = s_idc = s_bk = s_bkc = s_cnt = 0u;
@@ -135,11 +151,7 @@ __global__ void __launch_bounds__(256) k_merge_range(const uint32_t* in, long lo
             id = max(id, i); idc = max(idc, ~i); bk = max(bk, b); bkc = max(bkc, ~b);
             cnt++;
         }
-        key[j] = k;
-        amin[j] = 0xffffffffffffffffull;
-        if (LITE) pmin[j] = 0xffffffffu;
-        gor[j] = 0u;
-        gsum[j] = 0u;
+        if (key) key[j] = k;
     }
     const unsigned FULL = 0xffffffffu;
     id = __reduce_max_sync(FULL, id); idc = __reduce_max_sync(FULL, idc);
@@ -162,15 +174,18 @@ __device__ __forceinline__ uint32_t phx_merge_cell(const PhxMergeMap& m, unsigne
     return ((uint32_t)(k >> 48) - m.id0) * m.nbk + ((uint32_t)k - m.bk0);
 }
 
-// 2. the cells that occur
+// 2. the cells that occur; also clears the group slots
+template <int LITE>
 __global__ void __launch_bounds__(256) k_merge_present(const unsigned long long* key, long long n, const PhxMergeRange* range,
-                                                       unsigned long long most, uint32_t* cell)
+                                                       unsigned long long most, uint32_t* cell, unsigned long long* amin, uint32_t* pmin,
+                                                       uint32_t* gor, uint32_t* gsum)
 {
     const PhxMergeMap m = phx_merge_map(*range);
     if (m.cells == 0ull || m.cells > most) return;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
         const unsigned long long k = key[j];
+        phx_merge_clear<LITE>(j, amin, pmin, gor, gsum);
         if (k == PHX_MERGE_NONE) continue;
         const uint32_t c = phx_merge_cell(m, k);
         const uint32_t bit = 1u << (c & 31u);
@@ -275,16 +290,24 @@ __global__ void __launch_bounds__(256) k_merge_groups(const uint32_t* in, const 
 }
 
 // ---------------------------------------------------------------- sort form
+// record i is selected: by its key, where step 1 of the table form left one, or by its flags
+template <int LITE>
+__device__ __forceinline__ bool phx_merge_selected(const uint32_t* in, const unsigned long long* key, long long i, uint32_t mask)
+{
+    return key ? key[i] != PHX_MERGE_NONE : (in[i * PhxRec<LITE>::W + PhxRec<LITE>::FLAG] & mask) != 0u;
+}
+
 // 1a. per-tile selected counts
 template <int LITE>
-__global__ void __launch_bounds__(256) k_merge_sel_count(const uint32_t* in, long long n, uint32_t mask, uint32_t* tcount)
+__global__ void __launch_bounds__(256) k_merge_sel_count(const uint32_t* in, const unsigned long long* key, long long n, uint32_t mask,
+                                                          uint32_t* tcount)
 {
     __shared__ uint32_t wsum[8];
     const long long tile = (long long)blockIdx.x * PHX_MERGE_TILE;
     uint32_t c = 0;
     for (int r = 0; r < PHX_MERGE_TILE_ITEMS; r++) {
         const long long i = tile + (long long)r * 256 + threadIdx.x;
-        if (i < n) c += (in[i * PhxRec<LITE>::W + PhxRec<LITE>::FLAG] & mask) != 0u;
+        if (i < n) c += phx_merge_selected<LITE>(in, key, i, mask);
     }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = c;
@@ -296,10 +319,10 @@ __global__ void __launch_bounds__(256) k_merge_sel_count(const uint32_t* in, lon
     }
 }
 
-// 1b. ordered write of selected positions (tile offsets already scanned)
+// 1b. ordered write of selected positions, and of their keys where there are any (tile offsets already scanned)
 template <int LITE>
-__global__ void __launch_bounds__(256) k_merge_sel_write(const uint32_t* in, long long n, uint32_t mask, const uint32_t* toff,
-                                                          uint32_t* sel)
+__global__ void __launch_bounds__(256) k_merge_sel_write(const uint32_t* in, const unsigned long long* key, long long n, uint32_t mask,
+                                                          const uint32_t* toff, uint32_t* sel, unsigned long long* sel_key)
 {
     __shared__ uint32_t wsum[8];
     __shared__ uint32_t base;
@@ -309,13 +332,17 @@ __global__ void __launch_bounds__(256) k_merge_sel_write(const uint32_t* in, lon
     const long long tile = (long long)blockIdx.x * PHX_MERGE_TILE;
     for (int r = 0; r < PHX_MERGE_TILE_ITEMS; r++) {
         const long long i = tile + (long long)r * 256 + threadIdx.x;
-        const bool s = i < n && (in[i * PhxRec<LITE>::W + PhxRec<LITE>::FLAG] & mask) != 0u;
+        const bool s = i < n && phx_merge_selected<LITE>(in, key, i, mask);
         const uint32_t b = __ballot_sync(0xffffffffu, s);
         if (lane == 0) wsum[w] = __popc(b);
         __syncthreads();
         uint32_t before = base;
         for (int k = 0; k < w; k++) before += wsum[k];
-        if (s) sel[before + __popc(b & ((1u << lane) - 1u))] = (uint32_t)i;
+        if (s) {
+            const uint32_t p = before + __popc(b & ((1u << lane) - 1u));
+            sel[p] = (uint32_t)i;
+            if (sel_key) sel_key[p] = key[i];
+        }
         __syncthreads();
         if (threadIdx.x == 0) { uint32_t t = 0; for (int k = 0; k < 8; k++) t += wsum[k]; base += t; }
         __syncthreads();
@@ -336,14 +363,13 @@ __global__ void k_merge_gather(const uint32_t* in, const uint32_t* sel, long lon
     }
 }
 
-// 2. keys of the selected records
+// 2. keys of the selected records, where there is no room for the table form and so none yet
 template <int LITE>
-__global__ void k_merge_keys(const uint32_t* in, const uint32_t* sel, long long m, float tw, unsigned long long* key, uint32_t* val)
+__global__ void k_merge_keys(const uint32_t* in, const uint32_t* sel, long long m, float tw, unsigned long long* key)
 {
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (long long)gridDim.x * blockDim.x) {
         const long long i = sel ? (long long)sel[j] : j;
         key[j] = phx_merge_key<LITE>(in + i * PhxRec<LITE>::W, tw);
-        val[j] = (uint32_t)j;
     }
 }
 
@@ -362,7 +388,8 @@ __global__ void __launch_bounds__(256) k_radix_hist(const unsigned long long* ke
     hist[(size_t)threadIdx.x * ntile + blockIdx.x] = h[threadIdx.x];
 }
 
-// 3b. stable scatter: equal digits ranked by (round, warp, lane), i.e. by position in the tile
+// 3b. stable scatter: equal digits ranked by (round, warp, lane), i.e. by position in the tile (vin null: the
+// values are the positions)
 __global__ void __launch_bounds__(256) k_radix_scatter(const unsigned long long* kin, const uint32_t* vin, unsigned long long* kout,
                                                        uint32_t* vout, long long m, int shift, const uint32_t* off, int ntile)
 {
@@ -377,7 +404,7 @@ __global__ void __launch_bounds__(256) k_radix_scatter(const unsigned long long*
         const long long j = tile + (long long)r * 256 + t;
         const bool ok = j < m;
         const unsigned long long k = ok ? kin[j] : 0ull;
-        const uint32_t v = ok ? vin[j] : 0u;
+        const uint32_t v = !ok ? 0u : vin ? vin[j] : (uint32_t)j;
         const uint32_t d = ok ? ((uint32_t)(k >> shift) & 0xffu) : 0x100u;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
         const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
@@ -422,6 +449,13 @@ __global__ void k_scan_add(uint32_t* x, long long n, const uint32_t* tsum)
     if (i < n) x[i] += tsum[i / PHX_MERGE_SCAN_TILE];
 }
 
+template <int LITE>
+__global__ void k_merge_clear(long long ng, unsigned long long* amin, uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
+{
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < ng) phx_merge_clear<LITE>(g, amin, pmin, gor, gsum);
+}
+
 // 4a. group heads
 __global__ void k_merge_heads(const unsigned long long* key, long long m, uint32_t* head)
 {
@@ -429,11 +463,10 @@ __global__ void k_merge_heads(const unsigned long long* key, long long m, uint32
     if (j < m) head[j] = (j == 0 || key[j] != key[j - 1]) ? 1u : 0u;
 }
 
-// 4b. warp-segmented reduction per group, one atomic per (warp, group)
+// 4b. warp-segmented reduction per group, one atomic per (warp, group); val: input positions (null: 0, 1, ...)
 template <int LITE>
-__global__ void k_merge_reduce(const uint32_t* in, const uint32_t* sel, const unsigned long long* key, const uint32_t* val,
-                               const uint32_t* gexcl, long long m, unsigned long long* amin, uint32_t* pmin, uint32_t* gor,
-                               uint32_t* gsum)
+__global__ void k_merge_reduce(const uint32_t* in, const unsigned long long* key, const uint32_t* val, const uint32_t* gexcl,
+                               long long m, unsigned long long* amin, uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
 {
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -444,9 +477,8 @@ __global__ void k_merge_reduce(const uint32_t* in, const uint32_t* sel, const un
         if (ok) {
             const uint32_t head = (j == 0 || key[j] != key[j - 1]) ? 1u : 0u;
             g = gexcl[j] + head - 1u;
-            pos = val[j];
-            const long long i = sel ? (long long)sel[pos] : (long long)pos;
-            const uint32_t* r = in + i * PhxRec<LITE>::W;
+            pos = val ? val[j] : (uint32_t)j;
+            const uint32_t* r = in + (long long)pos * PhxRec<LITE>::W;
             tb = phx_time_order(r[PhxRec<LITE>::TIME]);
             fl = r[PhxRec<LITE>::FLAG];
             hc = r[PhxRec<LITE>::HC] >> 16;
@@ -459,7 +491,7 @@ __global__ void k_merge_reduce(const uint32_t* in, const uint32_t* sel, const un
         const uint32_t hs = __reduce_add_sync(peers, hc);
         if (ok && (__ffs(peers) - 1) == lane) {
             atomicMin(amin + g, ((unsigned long long)tmin << 32) | (unsigned long long)pfirst);
-            atomicMin(pmin + g, pm);
+            if (LITE) atomicMin(pmin + g, pm);
             atomicOr(gor + g, fo);
             atomicAdd(gsum + g, hs);
         }
@@ -468,14 +500,13 @@ __global__ void k_merge_reduce(const uint32_t* in, const uint32_t* sel, const un
 
 // 5. representative record per group with the reduced fields
 template <int LITE>
-__global__ void k_merge_write(const uint32_t* in, const uint32_t* sel, long long ng, const unsigned long long* amin,
-                              const uint32_t* pmin, const uint32_t* gor, const uint32_t* gsum, uint32_t* out)
+__global__ void k_merge_write(const uint32_t* in, long long ng, const unsigned long long* amin, const uint32_t* pmin,
+                              const uint32_t* gor, const uint32_t* gsum, uint32_t* out)
 {
     constexpr int W = PhxRec<LITE>::W;
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
-    const uint32_t pos = LITE ? pmin[g] : (uint32_t)(amin[g] & 0xffffffffull);
-    const long long i = sel ? (long long)sel[pos] : (long long)pos;
+    const long long i = LITE ? (long long)pmin[g] : (long long)(amin[g] & 0xffffffffull);
     uint32_t r[W];
     for (int w = 0; w < W; w++) r[w] = in[i * W + w];
     if (LITE) r[PhxRec<LITE>::TIME] = phx_time_unorder((uint32_t)(amin[g] >> 32));
