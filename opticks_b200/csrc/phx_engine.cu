@@ -1777,10 +1777,9 @@ static int launch_scan_t(int device, const PhxCsgCtx& csg, int root, float t_min
     return 0;
 }
 
-// Queries of at most this many rays take one thread per ray: 1,000 rays through the detector 24.7 us
-// against 28.1 as a stream, 100k 29.2 / 33.6, 200k 31.1 / 36.5, 500k 41.8 / 44.0; among bodies throughout the
-// volume 130k 78.5 / 79.9, 300k 143.1 / 135.7, with cones 20k 48.4 / 63.9, 300k 208.7 / 244.9.
-#define PHX_TRACE_EACH (1LL << 18)
+// A query whose rays all have a lane of one resident grid takes one thread per ray, a larger one the stream.
+// Rays anywhere in the detector, one thread per ray / stream: 1,000 29.4 / 33.4 us, 40k 45.7 / 52.3, 75k 45.9 /
+// 53.6 (75,776 lanes), 90k 59.2 / 55.5, 262k 103.5 / 67.3; polished (56,832 lanes) 40k 47.2 / 62.2, 60k 63.8 / 63.5.
 template <int CV>
 static int launch_trace_t(int device, const PhxScene& S, const float* d_rays, long long n, float t_min, float t_max, float4* out, unsigned* status,
                            cudaStream_t st)
@@ -1788,10 +1787,10 @@ static int launch_trace_t(int device, const PhxScene& S, const float* d_rays, lo
     static int grid[128] = {}, grid_each[128] = {};
     if (device < 0 || device >= 128) return phx_fail(-1, "device ordinal %d out of range", device);
     int rc;
-    if (n <= PHX_TRACE_EACH) {
-        if ((rc = wave_grid(k_trace_each<CV>, device, grid_each))) return rc;
-        const long long warps = 4LL * grid_each[device];            // few rays: narrower warps over all of them
-        const int width = (int)std::min<long long>(32, (n + warps - 1) / warps);
+    if ((rc = wave_grid(k_trace_each<CV>, device, grid_each))) return rc;
+    const long long warps = 4LL * grid_each[device];
+    if (n <= 32 * warps) {
+        const int width = (int)((n + warps - 1) / warps);           // few rays: narrower warps over all of them
         k_trace_each<CV><<<(unsigned)((n + 4 * width - 1) / (4 * width)), 128, 0, st>>>(S, d_rays, n, width, t_min, t_max, out, status);
         return 0;
     }

@@ -79,18 +79,19 @@ def test_one_thread_per_photon_equals_the_persistent_loop(cuda, name):
 @pytest.mark.parametrize("polish", [0, 1])
 @pytest.mark.parametrize("name", ["detector", "zoo", "sphere world", "with cones"])
 def test_trace_in_pieces(cuda, name, polish):
-    """a query of one ray more than the one-thread-per-ray rule takes (a stream of rays) against its pieces"""
+    """queries up to and beyond the lanes of one resident grid (148 SMs of 3 or 4 blocks of 128: one thread per ray
+    and the stream of rays) against queries of a few thousand"""
     from opticks_b200 import engine as E
     fd, phys, _ = SCENES[name](1)
     eng = E.Engine(fd.arrays(), phys, E.default_config(max_photon=64, root_polish=polish))
-    n = (1 << 18) + 1
+    n = 262_145
     rays = scenes.scan_rays(n, seed=5, half=11000.0 if name == "detector" else 1400.0)
-    whole, st = eng.trace(rays, 0.05)
-    assert st == 0
-    cuts = [0, 1, 1000, 1 << 17, n]
-    for a, b in zip(cuts, cuts[1:]):
-        piece, _ = eng.trace(np.ascontiguousarray(rays[:, a:b]), 0.05)
-        np.testing.assert_array_equal(piece.view(np.uint32), whole[a:b].view(np.uint32))
+    piece = 20_011
+    ref = np.concatenate([eng.trace(np.ascontiguousarray(rays[:, a:a + piece]), 0.05)[0] for a in range(0, n, piece)])
+    for m in (1, 31, 2369, 56_832, 56_833, 75_776, 75_777, n):
+        got, st = eng.trace(np.ascontiguousarray(rays[:, :m]), 0.05)
+        assert st == 0
+        np.testing.assert_array_equal(got.view(np.uint32), ref[:m].view(np.uint32))
     eng.close()
 
 
