@@ -756,8 +756,9 @@ def main():
                 "config": {"workload": "detector-17612pmt-scint-10M", "gensteps": len(gs), "photons_per_genstep": int(ppg),
                            "photons_per_step": N, "outputs": "photon+seq+hits(SD)+sensor counts",
                            "l2": "inputs larger than L2 (RNG states 240 MB read + 960 MB written per step)",
-                           "kernel": (f"wavefront: every photon of the event in flight, first bounces in the starting "
-                                      f"kernel, {rounds} rounds per step, then the tail kernel" if mode == 2 else
+                           "kernel": ("wavefront: every photon of the event in flight, " +
+                                      (f"{rounds} rounds" if rounds else "first bounces in the starting kernel") +
+                                      " per step, then the tail kernel" if mode == 2 else
                                       "persistent work queue, block 64, refill every bounce"),
                            "parallelism": f"{world} independent event streams" if world > 1 else "1 GPU"},
                 "gpu_launches": launches,

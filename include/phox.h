@@ -257,7 +257,8 @@ int phx_planck_icdf(float* out, int n);
 
 /* Diagnostics of the last phx_simulate / phx_simulate_device call on this engine (no reference
  * counterpart): kernels it launched and, in kernel_mode 2, wavefront rounds (one closest-hit and
- * one physics launch each) and, for phx_simulate_batched_device, whether it replayed a captured
+ * one physics launch each; 0 where the starting kernel took the first bounces or the call ran none,
+ * whatever wave_rounds says) and, for phx_simulate_batched_device, whether it replayed a captured
  * CUDA graph (*graph 1). */
 int phx_last_call_stats(phx_engine* e, int64_t* kernel_launches, int64_t* wave_rounds, int32_t* graph);
 

@@ -87,7 +87,9 @@ def tune_batched(engine, gs: np.ndarray, ev: np.ndarray, torch, reps: int = 2, s
 
 WAVE_REFILLS = (12,)
 WAVE_TAILS = (1 << 18,)                          # host-read schedule
-WAVE_ROUNDS = (2, 3, 4, 6, 8, 12, 16, 20)         # fixed schedule, graph-captured
+# fixed schedule, graph-captured: rounds, or, where the starting kernel takes the first bounces, half as many as
+# the bounces it takes (phx_config.wave_rounds)
+WAVE_ROUNDS = (2, 3, 4, 6, 8, 12, 16, 20)
 
 
 def tune_wavefront(engine, gs: np.ndarray, ev: np.ndarray, torch, reps: int = 1, sample_photons: int | None = None,

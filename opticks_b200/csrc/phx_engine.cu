@@ -1571,12 +1571,15 @@ static long long wave_pool_for(const phx_engine* e, long long N, bool adj)
     }
     return std::max<long long>(1, std::min(std::min(N, pool), PHX_WAVE_POOL_MAX));
 }
-// Scenes without such a ball: the rounds pay where many paths start coherently ahead of a hierarchy that the later bounces walk
-// divergently.  Calls of at most this many photons skip them: a round's two launches add more to the
-// longest path's latency than they save (detector events: 50k photons 217 us without rounds, 242 with
-// two; 200k 399 / 416; 500k 762 / 715).  So do calls on geometries without hierarchy leaves, whose
-// every bounce is coherent in the tail kernel's registers (1M torch photons in the sphere-in-box
-// 441-469 us, 556 with two rounds).
+// Calls of at most this many photons run no rounds: a round's two launches and the pool's traffic add more to
+// the longest path's latency than coherent first bounces save.  The line is that of a scene whose first
+// bounces are coherent (detector photons in rounds, without / with two: 50k 217 / 242 us, 200k 399 / 416, 500k
+// 762 / 715), which the starting kernel below has since taken over.  What is left for it are scenes without a
+// ball free of hierarchy leaves or with a global leaf that is not plain; among bodies throughout the volume
+// rounds cost at every size (20k 531 / 593 us, 200k 1,247 / 1,390, 300k 1,680 / 1,827, 1M 4,458 / 4,823), and
+// beyond the line they run because wave_rounds asks for them.  Calls on geometries without hierarchy
+// leaves run none either: every bounce is coherent in the tail kernel's registers (1M torch photons in the
+// sphere-in-box 441-469 us, 556 with two rounds).
 #define PHX_WAVE_SMALL 262144
 // Where the scene has plain global leaves and a ball free of hierarchy leaves, calls of at least this
 // many photons take their first 2 wave_rounds bounces in the starting kernel (k_wave_start) instead of

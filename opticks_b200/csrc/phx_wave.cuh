@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(128, ADJ ? 1 : PHX_WAVE_FILL_MINB) k_wave_init
 // would write and read the 128 B path and its 32 B PRD.  A path that must walk, or has taken `bounces`,
 // goes to its slot for the tail kernel.  For scenes whose globals are all plain.
 // Bound by the physics step's issue and the RNG state reads: 10M-photon detector event 10.2 -> 8.1 ms with
-// two bounces here instead of two rounds, 7.8 with four (one 9.5, three 7.8, six 7.9).  4 blocks per SM:
-// 96 registers without spills (5 blocks 8.11 ms, 6 blocks 8.24, 7 blocks 8.52, against 8.08).
+// two bounces here instead of two rounds, 7.8 with four (one 9.5, three 7.8, six 7.9).  4 blocks per SM asked
+// for: 90 registers, no spills, 5 blocks reside (a cap at 6 blocks 8.24 ms, at 7 8.52, against 8.08).
 #define PHX_WAVE_START_MINB 4
 template <bool POLISH>
 __global__ void __launch_bounds__(128, PHX_WAVE_START_MINB) k_wave_start(WaveArgs W, int bounces)
@@ -402,9 +402,10 @@ __global__ void __launch_bounds__(128, PHX_WAVE_START_MINB) k_wave_start(WaveArg
 // kernel takes 123 registers and the tail kernel 149: 4 blocks each, and 5 of the tail kernel for large
 // calls (10M photons: tail at 4 blocks 9.76 ms, 5 blocks 9.36, 6 blocks 9.87).  Small calls are the
 // latency of single paths, which the 5-block cap's spills lengthen (50k photons 200 us at 4 blocks, 211
-// at 5; 1M Cerenkov photons 1,167 and 1,150).  With the FP64 polish 3 blocks spill up to 390 B a thread: 2
-// (polished, among bodies of all kinds: 50k photons 1,423 -> 1,239 us, 1M 14.6 -> 13.9 ms).
-#define PHX_TRACE_MINB(cv) (((cv) & PHX_CV_PLAIN) != 0 ? 4 : PHX_CV_P(cv) ? 2 : 3)
+// at 5; 1M Cerenkov photons 1,167 and 1,150).  With the FP64 polish the tail kernel spills 340 B a thread at 3
+// blocks: 2 (polished, among bodies of all kinds: 50k photons 1,423 -> 1,239 us); the closest-hit kernels, with
+// as many spills, still gain by the third (1M polished rays through the detector 217.7 us at 2, 201.3 at 3).
+#define PHX_TRACE_MINB(cv) (((cv) & PHX_CV_PLAIN) != 0 ? 4 : 3)
 #define PHX_TAIL_MINB(cv, adj, wide) (!(adj) && ((cv) & PHX_CV_PLAIN) != 0 ? ((wide) ? 5 : 4) : PHX_CV_P(cv) ? 2 : 3)
 #define PHX_TAIL_WIDE (1LL << 19)       // photons of a call from which the 5-block tail kernel runs (with a hierarchy)
 
@@ -444,12 +445,13 @@ __global__ void __launch_bounds__(128, PHX_TRACE_MINB(CV)) k_wave_trace(WaveArgs
     if (status) atomicOr(W.A.status, status);
 }
 
-// The last live paths of a call, once few remain and no photons wait in the queue: persistent
-// warps run them to the end with the one-kernel loop's step (persist_step: the shared closest-hit
-// and physics code), so a long chain no longer costs two launches per bounce.  A lane whose path
-// ends takes the next one of the list at once (one atomic per warp on the round's ray counter,
-// which the physics kernel left at zero), so the lanes of a warp do not wait for its longest path.
-// Photons, seq and hits are the same as the rounds would give.
+// The paths of a call after its first bounces (of the starting kernel or of rounds; all of them in small calls),
+// or, host-read, the last live ones once few remain and no photons wait in the queue: persistent warps run
+// them to the end with the one-kernel loop's step (persist_step: the shared closest-hit and physics code),
+// without two launches and the pool's traffic per bounce; 60 % of a 10M-photon detector event.  A lane whose path
+// ends takes the next one of the list at once (one atomic per warp on the ray counter, which is zero
+// here: cleared with the call's counters, and by each round's physics kernel), so the lanes of a warp do not
+// wait for its longest path.  Photons, seq and hits are the same as the rounds would give.
 template <int CV, bool ADJ = false, bool WIDE = false>
 __global__ void __launch_bounds__(128, PHX_TAIL_MINB(CV, ADJ, WIDE)) k_wave_tail(WaveArgs W)
 {

@@ -1,4 +1,4 @@
-"""Every rule that picks a kernel or a variant by size, geometry or key range, at the edges where it turns:
+"""Rules that pick a kernel or a variant by size, geometry or key range, at the edges where they turn:
 spread and starting-kernel calls, the one-launch hit copy, the closest-hit kernels with and without
 the general evaluator, the scan's bounding ball, the event jump tables and the merge's key table."""
 import numpy as np

@@ -90,9 +90,9 @@ def test_wave_batched_equals_persistent(det, kw):
                                     dict(wave_rounds=10, use_graph=1, wave_refill=32),
                                     dict(wave_rounds=0, wave_tail=1 << 12, wave_refill=1)])
 def test_wave_schedules_equal_persistent(det, launch):
-    """the autotuner's knobs change no result: a fixed schedule of rounds then the tail kernel,
-    captured as a CUDA graph and replayed (second call), other refill thresholds, another tail
-    threshold; batched and plain calls"""
+    """the autotuner's knobs change no result: a fixed schedule (6 or 20 bounces in the starting kernel, then
+    the tail kernel), captured as a CUDA graph and replayed (second call), other refill thresholds, another
+    tail threshold; batched and plain calls"""
     torch = det[0]
     gs = scenes.batched_events(48, median=20000.0, lib=det[2])
     ev = np.arange(len(gs), dtype=np.int32)
