@@ -2634,8 +2634,9 @@ static int merge_impl(phx_engine* e, const uint32_t* in, long long n, uint32_t m
     }
     PHX_CU(room);
     k_merge_range<LITE><<<std::max(grid, 148u), 256, 0, st>>>(in, n, mask, tw, w.key0.p, w.range.p, w.cell.p, ncw);
-    k_merge_present<LITE><<<grid, 256, 0, st>>>(w.key0.p, n, w.range.p, most, w.cell.p, w.amin.p, w.pmin.p, w.gor.p, w.gsum.p);
-    k_merge_rank<<<(unsigned)nblk, 256, 0, st>>>(w.cell.p, w.range.p, most, w.cell_off.p, w.cell_blk.p);
+    k_merge_present<<<grid, 256, 0, st>>>(w.key0.p, n, w.range.p, most, w.cell.p);
+    k_merge_rank<LITE><<<(unsigned)nblk, 256, 0, st>>>(w.cell.p, w.range.p, most, w.cell_off.p, w.cell_blk.p, n, w.amin.p, w.pmin.p,
+                                                       w.gor.p, w.gsum.p);
     k_block_scan<<<1, 1024, 0, st>>>(w.cell_blk.p, (int)nblk, &w.range.p->groups);
     k_merge_fold<LITE><<<grid, 256, 0, st>>>(in, w.key0.p, n, w.range.p, most, w.cell.p, w.cell_off.p, w.cell_blk.p, w.amin.p, w.pmin.p,
                                              w.gor.p, w.gsum.p);

@@ -174,18 +174,15 @@ __device__ __forceinline__ uint32_t phx_merge_cell(const PhxMergeMap& m, unsigne
     return ((uint32_t)(k >> 48) - m.id0) * m.nbk + ((uint32_t)k - m.bk0);
 }
 
-// 2. the cells that occur; also clears the group slots
-template <int LITE>
+// 2. the cells that occur
 __global__ void __launch_bounds__(256) k_merge_present(const unsigned long long* key, long long n, const PhxMergeRange* range,
-                                                       unsigned long long most, uint32_t* cell, unsigned long long* amin, uint32_t* pmin,
-                                                       uint32_t* gor, uint32_t* gsum)
+                                                       unsigned long long most, uint32_t* cell)
 {
     const PhxMergeMap m = phx_merge_map(*range);
     if (m.cells == 0ull || m.cells > most) return;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
         const unsigned long long k = key[j];
-        phx_merge_clear<LITE>(j, amin, pmin, gor, gsum);
         if (k == PHX_MERGE_NONE) continue;
         const uint32_t c = phx_merge_cell(m, k);
         const uint32_t bit = 1u << (c & 31u);
@@ -193,11 +190,18 @@ __global__ void __launch_bounds__(256) k_merge_present(const unsigned long long*
     }
 }
 
-// 3. popcount prefix of the table, 1024 words a block (offsets within the block, block totals)
+// 3. popcount prefix of the table, 1024 words a block (offsets within the block, block totals); also clears the
+// group slots, where the table form goes on
+template <int LITE>
 __global__ void __launch_bounds__(256) k_merge_rank(const uint32_t* cell, const PhxMergeRange* range, unsigned long long most,
-                                                    uint32_t* off, uint32_t* blocksum)
+                                                    uint32_t* off, uint32_t* blocksum, long long n, unsigned long long* amin,
+                                                    uint32_t* pmin, uint32_t* gor, uint32_t* gsum)
 {
     const PhxMergeMap m = phx_merge_map(*range);
+    if (m.cells <= most) {
+        const long long stride = (long long)gridDim.x * blockDim.x;
+        for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += stride) phx_merge_clear<LITE>(g, amin, pmin, gor, gsum);
+    }
     const unsigned long long w0 = (unsigned long long)blockIdx.x * 1024ull;
     if (m.cells > most || w0 * 32ull >= m.cells) {
         if (threadIdx.x == 0) blocksum[blockIdx.x] = 0u;
